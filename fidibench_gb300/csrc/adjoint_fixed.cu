@@ -721,7 +721,8 @@ int adjoint_fixed_run(const AdjointFixedIO& io, cudaStream_t st) {
       for (int k = 1; k < len;) {
         const int kb = std::min(kRec, len - k);
         FDB_TRY(launch_fixed_one(g, c, fx::kR4W8S, kb, io.chain[cc], io.chain[cc ^ 1], false,
-                                 false, fr, pos, err, 0, kRec, logs + k, st, io.state_hi + k));
+                                 false, fr, pos, err, 0, kRec, logs + k, nullptr, st,
+                                 io.state_hi + k));
         cc ^= 1;
         ++pos;
         k += kb;

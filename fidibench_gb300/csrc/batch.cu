@@ -48,6 +48,7 @@
 #include <fstream>
 #include <sstream>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "step_fixed.cuh"
@@ -102,6 +103,7 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
   __shared__ int s_w;
   __shared__ int s_stop;
   __shared__ __align__(16) FixedArgs s_a;
+  __shared__ __align__(16) fx::LevelCoeffs s_lev;
 
   const long long total = (long long)nblocks * items_per_block;
   for (;;) {
@@ -127,6 +129,13 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
       const int* src = reinterpret_cast<const int*>(&I.a);
       int* dst = reinterpret_cast<int*>(&s_a);
       for (int k = threadIdx.x; k < (int)(sizeof(FixedArgs) / 4); k += blockDim.x) dst[k] = src[k];
+      // the coefficients of this block's levels: steps b K + 1 .. (b + 1) K
+      if (threadIdx.x < 3 * K) {
+        const int t = threadIdx.x / 3, j = threadIdx.x - 3 * t;
+        const QCoeff q = j == 0 ? I.a.qz : (j == 1 ? I.a.qy : I.a.qx);
+        const int n = b * K + t + 1;
+        s_lev.q[t][j] = step_qcoeff(q, n, n == steps);
+      }
     }
 
     // wait until every block b-1 tile of this instance is done
@@ -166,9 +175,18 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
     const int64_t* in = ((b & 1) ? arena1 : arena0) + I.offset;
     int64_t* out = ((b & 1) ? arena0 : arena1) + I.offset;
     unsigned long long my_or = 0ull;
-    fx::advance_tile<K, R, W, true, fx::kLoadL2Regs, false, false, true>(
-        s_a, 0, 0, 0, it.nout, levels, b == 0, b == nblocks - 1, s, d, in, out, s_dyn, s_row,
-        my_or, grp, lane - col * it.gw, (warp - rg * it.gh) * R);
+    // the last block holds the advect's last step, whose coefficients have all
+    // 62 bits; the same code for every block would cost the others the three
+    // products and the registers of a0
+    auto tile = [&](auto full) {
+      fx::advance_tile<K, R, W, true, fx::kLoadL2Regs, decltype(full)::value, false, false, true>(
+          s_a, s_lev, 0, 0, 0, it.nout, levels, b == 0, b == nblocks - 1, s, d, in, out, s_dyn,
+          s_row, my_or, grp, lane - col * it.gw, (warp - rg * it.gh) * R);
+    };
+    if (b == nblocks - 1)
+      tile(std::integral_constant<int, fx::kAllFull>{});
+    else
+      tile(std::integral_constant<int, fx::kNoneFull>{});
     fx::cta_or<W>(my_or, s_or, &sl[(b + 1) % 3].m);
     __threadfence();
     __syncthreads();

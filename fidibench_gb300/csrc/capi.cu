@@ -64,6 +64,7 @@ struct fdb_upwind {
   int chain_i = 0;
   int chain_first = 0;
   int chain_K = 0;
+  fdb::CoeffCarry chain_carry;  // coefficient errors carried from block to block
 };
 
 namespace fdb {
@@ -613,6 +614,7 @@ int fdb_upwind_block_begin(fdb_upwind* h, double dt, int* fixed) {
   h->arith_used = arith;
   h->chain_arith = arith;
   h->chain_first = 1;
+  h->chain_carry = CoeffCarry();
   if (arith == FDB_ARITH_FIXED) {
     h->chain_K = h->depth > 0 ? h->depth : default_depth(h->g);
     if (h->scale_slot < 0) {
@@ -638,7 +640,8 @@ int fdb_upwind_advect_block(fdb_upwind* h, int steps, double dt, int last) {
     if (steps > h->chain_K)
       return fail(FDB_ERR_INVALID, "a fixed-point block advances at most its depth of steps");
     rc = launch_fixed_block(h->g, c, steps, h->tune, h->chain_K, h->buf, &h->cur,
-                            h->chain_first != 0, last != 0, h->scratch, h->chain_i, h->stream);
+                            h->chain_first != 0, last != 0, h->scratch, h->chain_i,
+                            &h->chain_carry, h->stream);
     if (!rc) {
       ++h->chain_i;
       h->chain_first = 0;

@@ -147,6 +147,11 @@ struct FixedTuning {
   int tz = 0;      // output planes per CTA along z
 };
 
+// Coefficient errors carried from step to step of one fixed-point advect, per
+// internal axis (z, y, x), in units of 2^-62 (fixed_point.cuh).
+struct CoeffCarry {
+  int64_t r[3] = {0, 0, 0};
+};
 int launch_advect_fixed(const Geom& g, const Coeffs3& c, int steps, int depth,
                         double** buf, int* cur, double* d_scratch, size_t scratch_bytes,
                         cudaStream_t s);
@@ -161,11 +166,12 @@ int launch_advect_fixed_ex(const Geom& g, const Coeffs3& c, int steps, const Fix
 
 // One launch of a block chain (fdb_upwind_advect_block): k <= guard_K steps
 // at ring position i, FP64 in/out as asked, int64 otherwise; flips *cur.
+// carry is the chain's (zeros at its start).
 // The launches of a chain are those launch_advect_fixed_ex makes for the
 // same steps, so the field is the same bit for bit.
 int launch_fixed_block(const Geom& g, const Coeffs3& c, int k, const FixedTuning& tune,
                        int guard_K, double** buf, int* cur, bool in_f64, bool out_f64,
-                       double* d_scratch, int i, cudaStream_t s);
+                       double* d_scratch, int i, CoeffCarry* carry, cudaStream_t s);
 // The 64-bit word of ring slot i that the launch at position i reads to set
 // its scale (FP64 bits of max|f| after a pre-pass, else an OR of |F|).
 uint64_t* scale_word(double* d_scratch, int i);

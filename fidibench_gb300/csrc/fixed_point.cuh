@@ -20,6 +20,19 @@
 // when every D_j is zero.  Every product is
 // a 32 x 32 -> 64-bit multiply (IMAD.WIDE without an addend, which runs at
 // about twice the rate of the accumulating form on GB300).
+//
+// Within an advect of S steps only the last step needs all 62 bits of a_j.
+// The steps A_n = 1 + sum_j a_j,n D_j commute (constant coefficients, periodic
+// grid), so with a_j,n = a_j + e_j,n and sum_n e_j,n = 0
+//   prod_n A_n = A^S + O(sum_n e_n^2),
+// the first-order terms cancel whatever the order of the steps.  Steps 1 ..
+// S-1 therefore take the multiple of 2^-30 that carries the error of the steps
+// before it (dithered: |sum e| <= 2^-31 after every step), where a0 = 0 and
+// six products remain (fixed_update6), and step S takes the rest to 62 bits.
+// The remainder is S 2^-62 times a second difference of the field: below the
+// rounding of the S steps (2 units of F each), and the a0 d0 terms that the
+// nine-product form drops on every step (up to 6 units, with the sign of a0:
+// a drift of the mean) are dropped once.
 #pragma once
 
 #include <stdint.h>
@@ -111,6 +124,32 @@ inline QCoeff make_qcoeff(double a) {
   return q;
 }
 
+// The coefficient of step n >= 1 of an advect: q's nearest multiple of 2^-30
+// with the error of steps 1 .. n-1 carried in (a0 = 0), or to all 62 bits on
+// the last step.  n q.a0 - (C(n) << 32) in [-2^31, 2^31) is the error carried
+// past step n.
+FDB_HD QCoeff step_qcoeff(const QCoeff& q, int64_t n, bool last) {
+  const int64_t half = 0x80000000ll;
+  const int64_t before = ((n - 1) * (int64_t)q.a0 + half) >> 32;  // C(n - 1)
+  const int64_t after = (n * (int64_t)q.a0 + half) >> 32;         // C(n)
+  QCoeff r;
+  r.a1 = q.a1 + (int32_t)(after - before);
+  r.a0 = last ? (int32_t)(n * (int64_t)q.a0 - after * 0x100000000ll) : 0;
+  return r;
+}
+
+// The same step by step, for steps whose coefficient may change: *carry (0
+// before the first step) is the error carried in, in units of 2^-62.
+inline QCoeff step_qcoeff_carry(const QCoeff& q, int64_t* carry, bool last) {
+  const int64_t v = *carry + q.a0;
+  const int64_t inc = (v + 0x80000000ll) >> 32;
+  *carry = v - inc * 0x100000000ll;
+  QCoeff r;
+  r.a1 = q.a1 + (int32_t)inc;
+  r.a0 = last ? (int32_t)*carry : 0;
+  return r;
+}
+
 // 32 x 32 -> 64-bit products (one IMAD.WIDE each on the device)
 FDB_HD int64_t mulw_s(int32_t a, int32_t b) {
 #ifdef __CUDA_ARCH__
@@ -146,6 +185,21 @@ FDB_HD int64_t fixed_update_d(int64_t c, int64_t Dz, int64_t Dy, int64_t Dx, con
   const uint64_t lo2 = (uint64_t)(mulw_s(qz.a0, z1) + mulw_s(qy.a0, y1) + mulw_s(qx.a0, x1));
   const uint64_t lo = lo1 + lo2 + ((3ull << 59) + 0x80000000ull);
   const int64_t r = hi + (int64_t)(lo >> 32) - (3ll << 27);
+  return c + r * 4;
+}
+
+// fixed_update for coefficients with a0 = 0 (|F| <= 2^59 (1 + 2^-20) for the
+// cell and its upstream values): the same integer from six products, within 2
+// units of the exact F + sum_j a_j D_j.
+FDB_HD int64_t fixed_update6(int64_t c, int64_t zb, int64_t up, int64_t left, int32_t az,
+                             int32_t ay, int32_t ax) {
+  const int64_t Dz = zb - c, Dy = up - c, Dx = left - c;
+  const int64_t hi = mulw_s(az, (int32_t)(Dz >> 32)) + mulw_s(ay, (int32_t)(Dy >> 32)) +
+                     mulw_s(ax, (int32_t)(Dx >> 32));
+  // below 3 2^62 + 2^31: no overflow
+  const uint64_t lo = mulw_u((uint32_t)az, (uint32_t)Dz) + mulw_u((uint32_t)ay, (uint32_t)Dy) +
+                      mulw_u((uint32_t)ax, (uint32_t)Dx) + 0x80000000ull;
+  const int64_t r = hi + (int64_t)(lo >> 32);
   return c + r * 4;
 }
 

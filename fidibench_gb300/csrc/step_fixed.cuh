@@ -17,6 +17,13 @@ struct ScaleSlot {
 };
 
 constexpr int kMaxSlabs = 24;
+constexpr int kMaxDepth = 4;
+
+// Coefficients of the levels of one launch (z, y, x): level t takes step
+// number n0 + t of its advect (fixed_point.cuh step_qcoeff).
+struct LevelCoeffs {
+  QCoeff q[kMaxDepth][3];
+};
 
 struct FixedArgs {
   int nz, ny, nx;
@@ -28,6 +35,7 @@ struct FixedArgs {
   int nslab;
   int slab_z[kMaxSlabs + 1];
   QCoeff qz, qy, qx;
+  LevelCoeffs lev;  // per level (k_advect_fixed)
   int guard;
   const ScaleSlot* slot_in;
   ScaleSlot* slot_out;
@@ -72,12 +80,9 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// One level for one cell (fixed_point.cuh fixed_update: nine 32x32->64-bit
-// products, one rounding, exactly F when every difference is zero).
-__device__ __forceinline__ int64_t update(int64_t c, int64_t zb, int64_t up, int64_t left,
-                                          const FixedArgs& a) {
-  return fixed_update(c, zb, up, left, a.qz, a.qy, a.qx);
-}
+// Which levels of a launch take their coefficients to 62 bits (nine products
+// per cell); the others take 30 bits (six products).
+enum FullLevels { kNoneFull = 0, kLastFull = 1, kAllFull = 2 };
 
 // Dynamic shared memory of one CTA: plane prefetch [2][R][threads] (cp.async
 // loader only), plus the K-deep plane history [K][R][threads] when HSM.
@@ -151,9 +156,11 @@ struct TileGroup {
 // rectangle are its halo: the x-1 and y-1 neighbours they read from another
 // rectangle feed only halo cells, whose values are never stored.  tile_x,
 // tile_y and Z0 are unused, and every rectangle marches nout + K planes.
-template <int K, int R, int W, bool HSM, int LOADER, bool STORE_G = false,
+//
+// FULL: the levels whose coefficients in lev have a0 != 0.
+template <int K, int R, int W, bool HSM, int LOADER, int FULL, bool STORE_G = false,
           bool LEFT_SMEM = false, bool GROUPED = false>
-__device__ __forceinline__ void advance_tile(const FixedArgs& a, int tile_x, int tile_y, int Z0,
+__device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoeffs& lev, int tile_x, int tile_y, int Z0,
                                              int nout, int levels, bool in_f64, bool out_f64, int s, int d,
                                              const int64_t* __restrict__ in,
                                              int64_t* __restrict__ out, int64_t* s_dyn,
@@ -304,7 +311,11 @@ __device__ __forceinline__ void advance_tile(const FixedArgs& a, int tile_x, int
       }
       auto row = [&](int r, int64_t upv) {
         const int64_t c = cur[r];
-        const int64_t nv = update(c, HSM ? zb[r] : hist[HSM ? 0 : t][r], upv, left[r], a);
+        const int64_t zv = HSM ? zb[r] : hist[HSM ? 0 : t][r];
+        const QCoeff(&q)[3] = lev.q[t];
+        const int64_t nv = (FULL == kAllFull || (FULL == kLastFull && t == K - 1))
+                               ? fixed_update(c, zv, upv, left[r], q[0], q[1], q[2])
+                               : fixed_update6(c, zv, upv, left[r], q[0].a1, q[1].a1, q[2].a1);
         if (HSM) {
           if (!LEFT_SMEM) s_hist[t][r][tid] = c;
         } else {
@@ -399,9 +410,13 @@ k_advect_fixed(const int64_t* __restrict__ in, int64_t* __restrict__ out, const 
     }
   }
   unsigned long long my_or = 0ull;
-  advance_tile<K, R, W, HSM, LOAD, STORE_G, LEFT>(a, tile % a.tiles_x, tile / a.tiles_x, z0,
-                                                  nout, K, IN_F64, OUT_F64, s, d, in, out,
-                                                  s_dyn, s_row, my_or);
+  // the last level of an advect's last launch (the one that writes FP64), and
+  // every level of the adjoint's recompute, take 62-bit coefficients
+  constexpr int kFull = STORE_G ? kAllFull : (OUT_F64 ? kLastFull : kNoneFull);
+  advance_tile<K, R, W, HSM, LOAD, kFull, STORE_G, LEFT>(a, a.lev, tile % a.tiles_x,
+                                                         tile / a.tiles_x, z0, nout, K, IN_F64,
+                                                         OUT_F64, s, d, in, out, s_dyn, s_row,
+                                                         my_or);
   cta_or<W>(my_or, s_or, &a.slot_out->m);
 }
 
@@ -488,12 +503,15 @@ fx::FixedArgs make_fixed_args(const Geom& g, const Coeffs3& c, int shape, int K,
 int guard_bits(const Coeffs3& c, int K);
 // One launch of the single-field kernel (K steps, explicit buffers and slot
 // ring position i); scale_log (nullable, device) receives the output scale.
+// carry: the coefficient errors carried from the advect's earlier launches
+// (zeros before the first), updated; out_f64 marks its last launch.
 // gout (nullable; K arrays, int64 in and out, default shape only): every level
-// of the launch stored in state_g units, its scale in scale_log[0..K).
+// of the launch stored in state_g units, its scale in scale_log[0..K); every
+// level then takes the 62-bit coefficients and carry is not used.
 int launch_fixed_one(const Geom& g, const Coeffs3& c, int shape, int K, const void* in, void* out,
                      bool in_f64, bool out_f64, fx::ScaleSlot* slots, int i, int* err,
-                     int tz_override, int guard_K, int* scale_log, cudaStream_t st,
-                     int32_t* const* gout = nullptr);
+                     int tz_override, int guard_K, int* scale_log, CoeffCarry* carry,
+                     cudaStream_t st, int32_t* const* gout = nullptr);
 namespace fx {
 
 // defined in step_fixed_<shape>.cu; cap as in plan_slabs
