@@ -37,15 +37,15 @@
 // output tile of (32-K) x (R*W-K) cells in (x, y) and marches along z over tz
 // output planes after K warm-up planes.  Lanes are consecutive x (coalesced
 // 256 B row accesses), each thread holds R consecutive y rows of one column
-// in registers (shapes R x W = 8x8 and 4x16 with the plane history in
-// registers or shared memory, and 4x8 with it in shared memory, are
-// compiled).  Per level: x-1 from lane-1 by SHFL, y-1 from the thread's
-// previous row (row 0 from the warp above through shared memory, one
-// __syncthreads per level), z-1 from the thread's K-deep history of the
-// previous plane.  The next plane is prefetched with cp.async into shared
-// memory while the current one is computed.  The upstream halo (K columns,
-// K rows, K planes) is the only redundant work; periodic wrap is applied to
-// the coordinates of the loaded rows and planes.
+// in registers (R x W = 8x4 for all but small or thin grids, see
+// auto_config).  Per level: x-1 from lane-1 (its history slot, or SHFL), y-1
+// from the thread's previous row (row 0 from the warp above through shared
+// memory, one __syncthreads per level), z-1 from the thread's K-deep history
+// of the previous plane.  The next plane is loaded into registers (or, in the
+// older shapes, with cp.async into shared memory) while the current one is
+// computed.  The upstream halo (K columns, K rows, K planes) is the only
+// redundant work; periodic wrap is applied to the coordinates of the loaded
+// rows and planes.
 //
 // Scale protocol (no host synchronisation).  Three device slots hold
 // {m, s, kind}: kind 0 = m is the FP64 bit pattern of max|f| (from the
@@ -163,20 +163,16 @@ long long plan_slabs(FixedArgs& a, int resident, int cap) {
     return 0;
   }
   const long long res = resident > 0 ? resident : 1;
-  int h0 = cap;
-  if (h0 <= 0) {
-    h0 = (int)((txy * nz + 4 * res - 1) / (4 * res));
-    if (h0 < 32) h0 = 32;
-  }
-  if (h0 > nz) h0 = nz;
-  const int hmin = h0 < 8 ? h0 : 8;
+  constexpr int kMinPlanes = 8;
   int z = 0, i = 0;
   while (z < nz) {
     const int rem = nz - z;
+    const int left = kMaxSlabs - i;
     long long h = (txy * rem + res - 1) / res;  // remaining planes per resident CTA
-    if (h > h0) h = h0;
-    if (h < hmin) h = hmin;
-    if (h > rem || i == kMaxSlabs - 1) h = rem;
+    if (cap > 0 && h > cap) h = cap;
+    if (h < kMinPlanes && (cap <= 0 || cap >= kMinPlanes)) h = kMinPlanes;
+    if (h * left < rem) h = (rem + left - 1) / left;
+    if (h > rem) h = rem;
     a.slab_z[i++] = z;
     z += (int)h;
   }
@@ -210,8 +206,8 @@ int launch_fixed_one(const Geom& g, const Coeffs3& c, int shape, int K, const vo
     for (int j = 0; j < 3; ++j)
       a.lev.q[t][j] =
           gout ? q[j] : step_qcoeff_carry(q[j], &carry->r[j], out_f64 && t == K - 1);
-  // the grid is at most tiles_x * tiles_y * kMaxSlabs CTAs
-  if ((int64_t)a.tiles_x * a.tiles_y * fx::kMaxSlabs > 0x7FFFFFFF)
+  // the grid is at most tiles_x * tiles_y CTAs for each of min(nz, kMaxSlabs) slabs
+  if ((int64_t)a.tiles_x * a.tiles_y * (a.nz < fx::kMaxSlabs ? a.nz : fx::kMaxSlabs) > 0x7FFFFFFF)
     return fail(FDB_ERR_UNSUPPORTED, "grid too large for the fixed kernel");
   const int64_t* pin = (const int64_t*)in;
   int64_t* pout = (int64_t*)out;
@@ -230,6 +226,9 @@ int launch_fixed_one(const Geom& g, const Coeffs3& c, int shape, int K, const vo
     case fx::kR4W8S: fx::launch_r4w8s(K, in_f64, out_f64, cap, pin, pout, a, st); break;
     case fx::kR4W8L: fx::launch_r4w8l(K, in_f64, out_f64, cap, pin, pout, a, st); break;
     case fx::kR6W8L: fx::launch_r6w8l(K, in_f64, out_f64, cap, pin, pout, a, st); break;
+    case fx::kR8W4L: fx::launch_r8w4l(K, in_f64, out_f64, cap, pin, pout, a, st); break;
+    case fx::kR6W4L: fx::launch_r6w4l(K, in_f64, out_f64, cap, pin, pout, a, st); break;
+    case fx::kR4W4L: fx::launch_r4w4l(K, in_f64, out_f64, cap, pin, pout, a, st); break;
     default: fx::launch_r8w8(K, in_f64, out_f64, cap, pin, pout, a, st); break;
   }
   note_launch();
@@ -239,40 +238,67 @@ int launch_fixed_one(const Geom& g, const Coeffs3& c, int shape, int K, const vo
 
 namespace {
 
-// Default shape: 4 or 6 rows x 8 warps with the plane history in shared
-// memory, the next plane loaded into registers and the x-1 neighbour read
-// from the history.  Measured (advect(100), one GB300): 512^3 457 GCUPS for
-// 6 rows against 454 for 4 rows and 442 for the cp.async/shuffle 4 x 8 form;
-// 384^3 422 / 418 / 418; 320^3 416 / 395 / 391; 256^3 389 / 394 / 382.
-// Grids of up to 256^3 cells take 4 rows (more tiles keep the GPU full).
-int default_shape(const Geom& g, int K) {
-  (void)K;
-  return g.ntot > (uint64_t)256 * 256 * 256 ? fx::kR6W8L : fx::kR4W8L;
-}
-
-}  // namespace
-
-// Steps per launch for the default shape: the K that minimises the computed
-// tiles times the per-launch cost,
-//   ceil(nx / (32 - K)) * ceil(ny / (32 - K)) * (1 + 0.5 / K),
-// where 0.5 is the per-plane work (load, scale, store) in units of one
-// level's update (fitted to 160^3 .. 512^3 sweeps of K = 2..4, whose
-// winners this picks: 4 at 160, 3 at 256, 2 at 384, 3 at 512); ties go to
-// the deeper K.
-int default_depth(const Geom& g) {
-  int best = kMaxDepth;
+// The launch the automatic choice takes for g (depth K given, or 0: any).
+//
+// Shapes: 4 warps (one per SM sub-partition) of 8, 6 or 4 rows, the plane
+// history in shared memory.  Few warps with many rows win: a level's barrier
+// waits for 4 warps instead of 8, and 8 independent rows per thread hide the
+// latency of the products better than more warps do.  Measured (inner launch,
+// K = 3, GCUPS, 8x4 / 6x8 / 4x8 / 8x8): 512^3 610 / 572 / 547 / 571; 256^3
+// 502 / 482 / 464 / 440.
+//
+// A launch of K steps costs the computed tiles (32 columns x R W rows, of which
+// 32 - K and R W - K are output) times K levels plus the per-plane work (load,
+// scale, store), 0.86 levels, per step: minimal
+//   ceil(nx / (32 - K)) ceil(ny / (R W - K)) R W (1 + 0.86 / K) f(R)
+// with f the measured cost of a computed row against 8 rows per thread.  It
+// picks the winners of a sweep over 64^3 .. 512^3 and uneven grids, or within
+// 7 % of them (winner's K: 4 at 128, 192, 384, 448; 3 at 256, 288, 512).
+// Grids whose 8-row tiles give less than half a wave of CTAs (8 planes each)
+// are bound by the latency of a CTA's march: 4 rows (more CTAs) and K = 4
+// (64^3: 94 against 85 GCUPS for 8 rows).
+struct Config {
+  int K, shape;
+};
+Config auto_config(const Geom& g, int K_asked) {
+  struct Cand {
+    int shape;
+    double f;
+  };
+  static const Cand cands[] = {{fx::kR8W4L, 1.0}, {fx::kR6W4L, 1.02}, {fx::kR4W4L, 1.1}};
+  const int K_hi = K_asked > 0 ? K_asked : kMaxDepth;
+  const int K_lo = K_asked > 0 ? K_asked : 2;
+  const auto tiles = [&](int K, int rows) {
+    return std::ceil((double)g.nx / (32 - K)) * std::ceil((double)g.ny / (rows - K));
+  };
+  constexpr double kHalfWave = 152 * 4 / 2;  // CTAs
+  if (tiles(K_hi, 32) * std::ceil(g.nz / 8.0) < kHalfWave) return {K_hi, fx::kR4W4L};
+  Config best{K_hi, fx::kR8W4L};
   double best_cost = 0.0;
-  for (int K = kMaxDepth; K >= 2; --K) {
-    const double w = 32.0 - K;
-    const double tiles = std::ceil(g.nx / w) * std::ceil(g.ny / w);
-    const double cost = tiles * (1.0 + 0.5 / K);
-    if (K == kMaxDepth || cost < best_cost) {
-      best = K;
-      best_cost = cost;
+  for (int K = K_hi; K >= K_lo; --K) {
+    for (const Cand& c : cands) {
+      const int rows = fx::shape_rows(c.shape) * fx::shape_warps(c.shape);
+      const double cost = tiles(K, rows) * rows * (1.0 + 0.86 / K) * c.f;
+      if (best_cost == 0.0 || cost < best_cost) {
+        best_cost = cost;
+        best = {K, c.shape};
+      }
     }
   }
   return best;
 }
+
+// The shape of a launch of k <= K steps in an advect of depth K.  One step per
+// launch is conversion work for the most part, with few chains to overlap:
+// 4 rows at 6 CTAs per SM (advect(1) at 256^3, FP64 in and out: 161 GCUPS
+// against 144 for 8 rows).
+int default_shape(const Geom& g, int K, int k) {
+  return k == 1 ? (int)fx::kR4W4L : auto_config(g, K).shape;
+}
+
+}  // namespace
+
+int default_depth(const Geom& g) { return auto_config(g, 0).K; }
 
 int fixed_supported(const Geom& g, const Coeffs3& c, int depth) {
   if (g.ndims > 3) return fail(FDB_ERR_UNSUPPORTED, "fixed kernel serves ndims <= 3");
@@ -325,8 +351,9 @@ int launch_fixed_block(const Geom& g, const Coeffs3& c, int k, const FixedTuning
                        int guard_K, double** buf, int* cur, bool in_f64, bool out_f64,
                        double* d_scratch, int i, CoeffCarry* carry, cudaStream_t s) {
   if (fault_injected("launch")) return fail(FDB_ERR_INJECTED, "injected launch failure");
-  const int shape =
-      (tune.shape >= 0 && tune.shape < fx::kNumShapes) ? tune.shape : default_shape(g, guard_K);
+  const int shape = (tune.shape >= 0 && tune.shape < fx::kNumShapes)
+                        ? tune.shape
+                        : default_shape(g, guard_K, k);
   FDB_TRY(launch_fixed_one(g, c, shape, k, buf[*cur], buf[*cur ^ 1], in_f64, out_f64,
                            (ScaleSlot*)d_scratch, i, fixed_error_word(d_scratch), tune.tz, guard_K,
                            nullptr, carry, s));
@@ -355,8 +382,7 @@ int launch_advect_fixed_ex(const Geom& g, const Coeffs3& c, int steps, const Fix
   ScaleSlot* slots = (ScaleSlot*)d_scratch;
   int* err = fixed_error_word(d_scratch);
   const int K = tune.depth > 0 ? tune.depth : default_depth(g);
-  const int shape =
-      (tune.shape >= 0 && tune.shape < fx::kNumShapes) ? tune.shape : default_shape(g, K);
+  const bool shape_set = tune.shape >= 0 && tune.shape < fx::kNumShapes;
   int i0 = (scale_slot && *scale_slot >= 0) ? *scale_slot : -1;
   if (i0 < 0) {
     FDB_TRY(launch_scale_prepass(g, buf[*cur], d_scratch, s));
@@ -367,6 +393,7 @@ int launch_advect_fixed_ex(const Geom& g, const Coeffs3& c, int steps, const Fix
   CoeffCarry carry;
   for (int l = 0, done = 0; l < nlaunch; ++l, ++i) {
     const int k = (steps - done) < K ? (steps - done) : K;
+    const int shape = shape_set ? tune.shape : default_shape(g, K, k);
     FDB_TRY(launch_fixed_one(g, c, shape, k, buf[*cur], buf[*cur ^ 1], l == 0, l == nlaunch - 1,
                              slots, i, err, tune.tz, K, nullptr, &carry, s));
     *cur ^= 1;

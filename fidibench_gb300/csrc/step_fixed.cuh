@@ -16,7 +16,7 @@ struct ScaleSlot {
   int kind;
 };
 
-constexpr int kMaxSlabs = 24;
+constexpr int kMaxSlabs = 64;
 constexpr int kMaxDepth = 4;
 
 // Coefficients of the levels of one launch (z, y, x): level t takes step
@@ -423,20 +423,30 @@ k_advect_fixed(const int64_t* __restrict__ in, int64_t* __restrict__ out, const 
 // Kernel shapes compiled into the library: rows per thread x warps per CTA,
 // history in registers (reg) or shared memory (smem); the L shapes load the
 // next plane into registers and take the x-1 neighbour from the history
-// (kLoadRegs, LEFT_SMEM).
+// (kLoadRegs, LEFT_SMEM).  The first kNumShapes can be asked for; the 4-warp
+// shapes past them are what the automatic choice takes (step_fixed.cu
+// auto_config).
 enum Shape {
   kR8W8 = 0, kR4W16 = 1, kR8W8S = 2, kR4W16S = 3, kR4W8S = 4, kR4W8L = 5, kR6W8L = 6,
-  kNumShapes = 7
+  kNumShapes = 7,
+  kR8W4L = 7, kR6W4L = 8, kR4W4L = 9
 };
 constexpr int shape_rows(int sh) {
-  return (sh == kR8W8 || sh == kR8W8S) ? 8 : (sh == kR6W8L ? 6 : 4);
+  return (sh == kR8W8 || sh == kR8W8S || sh == kR8W4L) ? 8
+         : (sh == kR6W8L || sh == kR6W4L)              ? 6
+                                                       : 4;
 }
-constexpr int shape_warps(int sh) { return (sh == kR4W16 || sh == kR4W16S) ? 16 : 8; }
+constexpr int shape_warps(int sh) {
+  return (sh == kR4W16 || sh == kR4W16S) ? 16 : (sh >= kR8W4L ? 4 : 8);
+}
 
 // z-slabs of one k_advect_fixed launch for `resident` CTAs on the GPU at once:
-// slabs of h0 planes (cap if > 0, else about a quarter of the planes per
-// resident CTA, at least 32), then slabs that follow the remaining planes per
-// resident CTA down to 8.  Sets a.nslab / a.slab_z; returns the CTA count.
+// every slab takes the remaining planes per resident CTA (at most cap if > 0),
+// at least 8 and as many as kMaxSlabs slabs need.  The first slabs fill the
+// GPU once with the longest runs (K warm-up planes per slab), the short last
+// ones even out the end.  Measured (512^3, K = 3, 8 x 4): 617 GCUPS against 609
+// for first slabs of a quarter of that height; 256^3 509 against 502.  Sets
+// a.nslab / a.slab_z; returns the CTA count.
 long long plan_slabs(FixedArgs& a, int resident, int cap);
 
 template <int K, int R, int W, bool HSM, int MINB, bool IN, bool OUT, bool STORE_G = false,
@@ -528,6 +538,9 @@ FDB_FX_DECLARE(launch_r4w16s)
 FDB_FX_DECLARE(launch_r4w8s)
 FDB_FX_DECLARE(launch_r4w8l)
 FDB_FX_DECLARE(launch_r6w8l)
+FDB_FX_DECLARE(launch_r8w4l)
+FDB_FX_DECLARE(launch_r6w4l)
+FDB_FX_DECLARE(launch_r4w4l)
 #undef FDB_FX_DECLARE
 
 }  // namespace fx
