@@ -290,8 +290,8 @@ Config auto_config(const Geom& g, int K_asked) {
 
 // The shape of a launch of k <= K steps in an advect of depth K.  One step per
 // launch is conversion work for the most part, with few chains to overlap:
-// 4 rows at 6 CTAs per SM (advect(1) at 256^3, FP64 in and out: 161 GCUPS
-// against 144 for 8 rows).
+// 4 rows at 6 CTAs per SM (advect(1) at 256^3, FP64 in and out: 194 GCUPS
+// against 175 for 8 rows).
 int default_shape(const Geom& g, int K, int k) {
   return k == 1 ? (int)fx::kR4W4L : auto_config(g, K).shape;
 }
