@@ -82,6 +82,8 @@ SIGNATURES: dict[str, tuple] = {
     "fdb_batch_set_velocity": (_int, [_vp, _int, _vp]),
     "fdb_batch_set_field": (_int, [_vp, _int, _vp, _int]),
     "fdb_batch_get_field": (_int, [_vp, _int, _vp, _int]),
+    "fdb_batch_set_fields": (_int, [_vp, _vp, _int]),
+    "fdb_batch_get_fields": (_int, [_vp, _vp, _int]),
     "fdb_batch_init_sphere": (_int, [_vp, _int, _vp, ctypes.c_double, ctypes.c_double,
                                      ctypes.c_uint64]),
     "fdb_batch_set_stream": (_int, [_vp, _vp]),

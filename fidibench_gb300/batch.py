@@ -180,10 +180,7 @@ class Batch:
             if values.size != total:
                 raise ValueError(f"need {total} values, got {values.size}")
             base = values.ctypes.data
-        off = 0
-        for k, n in enumerate(self.sizes):
-            check(lib.fdb_batch_set_field(self._h, k, base + 8 * off, 1 if dev else 0))
-            off += n
+        check(lib.fdb_batch_set_fields(self._h, base, 1 if dev else 0))
 
     def get_fields(self, out=None):
         """All fields into one concatenated array (numpy, or `out`: a numpy
@@ -197,10 +194,7 @@ class Batch:
         if not dev and out.size != total:
             raise ValueError(f"need {total} values")
         base = out.data_ptr() if dev else out.ctypes.data
-        off = 0
-        for k, n in enumerate(self.sizes):
-            check(lib.fdb_batch_get_field(self._h, k, base + 8 * off, 1 if dev else 0))
-            off += n
+        check(lib.fdb_batch_get_fields(self._h, base, 1 if dev else 0))
         return out
 
     def set_velocity(self, index: int, velocity) -> None:

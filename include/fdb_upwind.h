@@ -321,6 +321,11 @@ int fdb_batch_count(fdb_batch* b, int* count, uint64_t* total_cells);
 int fdb_batch_storage_order(fdb_batch* b, int index, int* order3);
 int fdb_batch_set_field(fdb_batch* b, int index, const double* src, int is_device);
 int fdb_batch_get_field(fdb_batch* b, int index, double* dst, int is_device);
+/* All instances' fields at once, one after another in the caller's order
+ * (instance i starts at the sum of the sizes before it); device fields move in
+ * one launch. */
+int fdb_batch_set_fields(fdb_batch* b, const double* src, int is_device);
+int fdb_batch_get_fields(fdb_batch* b, double* dst, int is_device);
 int fdb_batch_init_sphere(fdb_batch* b, int index, const double* center, double radius,
                           double noise_amp, uint64_t seed);
 int fdb_batch_set_stream(fdb_batch* b, void* cuda_stream);
