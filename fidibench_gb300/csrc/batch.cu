@@ -90,9 +90,12 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 }
 
 // 4-row shapes: at least 32 warps per SM (64 registers per thread, no
-// spills); 8-row shapes: 16 warps (their rows need the registers)
-template <int K, int R, int W>
-__global__ void __launch_bounds__(32 * W, (R > 4 ? 512 : 1024) / (32 * W))
+// spills); 6-row shapes: 20 warps, 8-row shapes: 16 warps (their rows need the
+// registers).  kLeft: the x - 1 neighbour from the plane history (LEFT_SMEM of
+// advance_tile), which the 4-warp shapes take and the 64-register ones do not
+// (slower there).
+template <int K, int R, int W, bool kLeft>
+__global__ void __launch_bounds__(32 * W, (R > 6 ? 512 : R > 4 ? 640 : 1024) / (32 * W))
 k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ items,
               const fx::TileGroup* __restrict__ groups, int items_per_block, int nblocks,
               int steps, int64_t* arena0, int64_t* arena1, ScaleSlot* slots, unsigned* done,
@@ -171,22 +174,21 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
     const int col = min(lane / it.gw, ncol - 1);
     const int rg = min(warp / it.gh, nrow - 1);
     const fx::TileGroup grp = groups[it.group_base + rg * ncol + col];
-    const int levels = min(K, steps - b * K);
     const int64_t* in = ((b & 1) ? arena1 : arena0) + I.offset;
     int64_t* out = ((b & 1) ? arena0 : arena1) + I.offset;
     unsigned long long my_or = 0ull;
     // the last block holds the advect's last step, whose coefficients have all
     // 62 bits; the same code for every block would cost the others the three
     // products and the registers of a0
-    auto tile = [&](auto full) {
-      fx::advance_tile<K, R, W, true, fx::kLoadL2Regs, decltype(full)::value, false, false, true>(
-          s_a, s_lev, 0, 0, 0, it.nout, levels, b == 0, b == nblocks - 1, s, d, in, out, s_dyn,
-          s_row, my_or, grp, lane - col * it.gw, (warp - rg * it.gh) * R);
+    auto tile = [&](auto full, int levels, bool out_f64) {
+      fx::advance_tile<K, R, W, true, fx::kLoadL2Regs, decltype(full)::value, false, kLeft, true>(
+          s_a, s_lev, 0, 0, 0, it.nout, levels, b == 0, out_f64, s, d, in, out, s_dyn, s_row,
+          my_or, grp, lane - col * it.gw, (warp - rg * it.gh) * R);
     };
     if (b == nblocks - 1)
-      tile(std::integral_constant<int, fx::kAllFull>{});
+      tile(std::integral_constant<int, fx::kAllFull>{}, steps - b * K, true);
     else
-      tile(std::integral_constant<int, fx::kNoneFull>{});
+      tile(std::integral_constant<int, fx::kNoneFull>{}, K, false);
     fx::cta_or<W>(my_or, s_or, &sl[(b + 1) % 3].m);
     __threadfence();
     __syncthreads();
@@ -494,7 +496,7 @@ std::array<int, 3> choose_order(const uint64_t n[3]) {
   return best;
 }
 
-template <int K, int R, int W>
+template <int K, int R, int W, bool kLeft = false>
 int launch_batch_kernel(int grid, const InstDev* insts, const ItemDev* items,
                         const fx::TileGroup* groups, int ipb, int nblocks, int steps, int64_t* a0,
                         int64_t* a1, ScaleSlot* slots, unsigned* done, unsigned* queue, int* err,
@@ -502,22 +504,22 @@ int launch_batch_kernel(int grid, const InstDev* insts, const ItemDev* items,
   constexpr int smem = K * R * 32 * W * (int)sizeof(int64_t);
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(k_batch_fixed<K, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_batch_fixed<K, R, W, kLeft>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          smem);
     configured = true;
   }
-  k_batch_fixed<K, R, W><<<grid, 32 * W, smem, st>>>(insts, items, groups, ipb, nblocks, steps,
+  k_batch_fixed<K, R, W, kLeft><<<grid, 32 * W, smem, st>>>(insts, items, groups, ipb, nblocks, steps,
                                                      a0, a1, slots, done, queue, err, wait_bias,
                                                      wait_cycles);
   return FDB_OK;
 }
 
-template <int K, int R, int W>
+template <int K, int R, int W, bool kLeft = false>
 int resident_ctas_of() {
   constexpr int smem = K * R * 32 * W * (int)sizeof(int64_t);
-  cudaFuncSetAttribute(k_batch_fixed<K, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_batch_fixed<K, R, W, kLeft>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_fixed<K, R, W>, 32 * W, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_fixed<K, R, W, kLeft>, 32 * W, smem);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -547,6 +549,9 @@ const Variant kVariants[] = {
     {2, fx::kR8W8S, launch_batch_kernel<2, 8, 8>, resident_ctas_of<2, 8, 8>},
     {3, fx::kR8W8S, launch_batch_kernel<3, 8, 8>, resident_ctas_of<3, 8, 8>},
     {4, fx::kR8W8S, launch_batch_kernel<4, 8, 8>, resident_ctas_of<4, 8, 8>},
+    // by the automatic choice only
+    {2, fx::kR6W4L, launch_batch_kernel<2, 6, 4, true>, resident_ctas_of<2, 6, 4, true>},
+    {3, fx::kR6W4L, launch_batch_kernel<3, 6, 4, true>, resident_ctas_of<3, 6, 4, true>},
 };
 
 const Variant* find_variant(int K, int shape) {
@@ -609,8 +614,9 @@ struct fdb_batch {
   IoDev* d_io = nullptr;              // k_batch_io's table (null: too many work items)
   uint32_t io_items = 0;
   cudaStream_t own = nullptr, stream = nullptr;
-  // tuning (0 / -1 = automatic)
+  // tuning as set (0 / -1 = automatic), and what the launches take
   int K = 0, shape = -1, tz = 0;
+  int eff_K = 0, eff_shape = -1, eff_tz = 0;
   // graph cache
   cudaGraphExec_t graph = nullptr;
   std::string graph_key;
@@ -859,7 +865,65 @@ int run_looped(fdb_batch* b, int steps, const double* dt, int K) {
   return FDB_OK;
 }
 
-int effective_K(fdb_batch* b) { return b->K > 0 ? b->K : kDefaultDepth; }
+// Fills in the tuning that is not set (b->eff_*).
+//
+// Depth 2 or 3 and CTAs of 4 rows x 8 warps or 6 rows x 4 warps: the fewest
+// computed rows, sum over the packed tiles of (planes + K) R W (K + 0.86) / K
+// (0.86 levels: a plane's load, scale and store), as in the single-field
+// choice.  Ranges of z: few long tiles per time block leave CTAs idle until
+// the block's last tile is done, short ones repeat K warm-up planes each.
+// With q the tile-planes of a block per resident CTA, 3 sqrt(q) + q / 30 planes
+// (at least 8) is within 7 % of the best of a sweep (12 .. 200 instances, q from 3
+// to 340); from q = 400 on whole columns are best.  Measured, advect GCUPS,
+// depth 2, 4 rows and whole columns -> this: 8 x 96^3 99 -> 271; 40 x 64^3
+// 200 -> 375; 33 instances of [61, 98]^3 211 -> 349; 64 x 128^3 465 -> 496.
+void choose_tuning(fdb_batch* b) {
+  struct Cand {
+    int K, shape;
+  };
+  static const Cand cands[] = {
+      {2, fx::kR4W8S}, {3, fx::kR4W8S}, {2, fx::kR6W4L}, {3, fx::kR6W4L}};
+  std::vector<Cand> list;
+  for (const Cand& c : cands)
+    if ((b->K <= 0 || b->K == c.K) && (b->shape < 0 || b->shape == c.shape)) list.push_back(c);
+  // a setting outside the candidates: itself, the rest at their first choice
+  if (list.empty())
+    list.push_back({b->K > 0 ? b->K : kDefaultDepth, b->shape >= 0 ? b->shape : (int)fx::kR4W8S});
+  auto pack = [&](const Cand& c, int tz, std::vector<ItemDev>* items) {
+    std::vector<fx::TileGroup> groups;
+    items->clear();
+    for (int i = 0; i < b->count; ++i) {
+      const Geom& g = b->geoms[i];
+      pack_instance((int)g.nx, (int)g.ny, (int)g.nz, i, c.K, fx::shape_rows(c.shape),
+                    fx::shape_warps(c.shape), tz, items, &groups);
+    }
+  };
+  double best = 0.0;
+  std::vector<ItemDev> items;
+  for (const Cand& c : list) {
+    int tz = b->tz;
+    if (tz <= 0) {
+      const Variant* v = find_variant(c.K, c.shape);
+      pack(c, 0, &items);
+      double planes = 0.0;
+      for (const ItemDev& it : items) planes += it.nout;
+      const double q = planes / (v ? v->resident() : 1);
+      tz = q >= 400.0 ? 0 : std::max(8, (int)ceil(3.0 * sqrt(q) + q / 30.0));
+    }
+    pack(c, tz, &items);
+    double cost = 0.0;
+    for (const ItemDev& it : items) cost += it.nout + c.K;
+    cost *= fx::shape_rows(c.shape) * fx::shape_warps(c.shape) * (1.0 + 0.86 / c.K);
+    if (best == 0.0 || cost < best) {
+      best = cost;
+      b->eff_K = c.K;
+      b->eff_shape = c.shape;
+      b->eff_tz = tz;
+    }
+  }
+}
+
+int effective_K(fdb_batch* b) { return b->eff_K; }
 
 void free_batch_adjoint(fdb_batch* b) {
   for (double* p : b->adj_ckpt) cudaFree(p);
@@ -970,7 +1034,9 @@ int io_all(fdb_batch* b, const double* src, double* dst, bool to_view) {
   return FDB_OK;
 }
 
-int effective_shape(fdb_batch* b) { return b->shape >= 0 ? b->shape : fx::kR4W8S; }
+int effective_shape(fdb_batch* b) { return b->eff_shape; }
+
+int effective_tz(fdb_batch* b) { return b->eff_tz; }
 
 }  // namespace
 
@@ -1057,6 +1123,7 @@ int fdb_batch_create(int count, const fdb_instance_desc* descs, fdb_batch** out)
     fdb_batch_destroy(b);
     return cuda_fail(e, "batch set-up");
   }
+  choose_tuning(b);
   rc = make_io_table(b);
   // each instance starts like the reference constructor: f = 0, f[0] = 1
   for (int i = 0; i < count && !rc; ++i)
@@ -1224,6 +1291,7 @@ int fdb_batch_set_tuning(fdb_batch* b, int key, int value) {
   } else {
     return fail(FDB_ERR_INVALID, "unknown tuning key");
   }
+  choose_tuning(b);
   drop_graph(b);
   return FDB_OK;
 }
@@ -1234,7 +1302,7 @@ int fdb_batch_advect(fdb_batch* b, int num_steps, const double* dt) {
   if (num_steps < 0) return fail(FDB_ERR_INVALID, "num_steps must be >= 0");
   FDB_TRY(check_dts(b, dt));
   if (num_steps == 0) return FDB_OK;
-  const int rc = run_batched(b, num_steps, dt, effective_K(b), effective_shape(b), b->tz, true);
+  const int rc = run_batched(b, num_steps, dt, effective_K(b), effective_shape(b), effective_tz(b), true);
   if (rc == FDB_ERR_UNSUPPORTED) {
     // some instance is outside the fixed kernel's domain: loop the plain path
     return run_looped(b, num_steps, dt, effective_K(b));
@@ -1285,7 +1353,7 @@ static int batch_lam_steps(fdb_batch* b, int S, const double* dt, int* lc) {
   std::swap(b->arena[1], b->adj_lam[1]);
   b->cur = *lc;
   b->transposed_run = true;
-  const int rc = run_batched(b, S, dt, effective_K(b), effective_shape(b), b->tz, false);
+  const int rc = run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b), false);
   *lc = b->cur;
   std::swap(b->arena[0], b->adj_lam[0]);
   std::swap(b->arena[1], b->adj_lam[1]);
@@ -1347,7 +1415,7 @@ static int batch_adjoint_closed_form(fdb_batch* b, int S, const double* dt,
   FDB_TRY(batch_lam_steps(b, 1, dt, &lc));
   FDB_TRY(batch_lam_store(b, lc, grad_f0, is_device));
   if (advance_fields)
-    FDB_TRY(run_batched(b, S, dt, effective_K(b), effective_shape(b), b->tz, true));
+    FDB_TRY(run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b), true));
   std::vector<double> dda(3 * (size_t)n);
   FDB_CUDA_TRY(cudaMemcpyAsync(dda.data(), b->adj_dda, dda.size() * 8, cudaMemcpyDeviceToHost,
                                b->stream));
@@ -1362,7 +1430,7 @@ static int batch_adjoint_closed_form(fdb_batch* b, int S, const double* dt,
 static int batch_adjoint_f0_only(fdb_batch* b, int S, const double* dt, const double* lambda_T,
                                  double* grad_f0, int is_device) {
   if (S > 0 && b->adj_mode != 2)  // form 2 keeps the fields at f0
-    FDB_TRY(run_batched(b, S, dt, effective_K(b), effective_shape(b), b->tz, true));
+    FDB_TRY(run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b), true));
   return batch_transposed(b, S, dt, lambda_T, grad_f0, is_device);
 }
 
@@ -1448,7 +1516,7 @@ int fdb_batch_adjoint(fdb_batch* b, int num_steps, const double* dt, const doubl
     FDB_CUDA_TRY(cudaMemcpyAsync(b->adj_ckpt[sg], b->arena[b->cur], T * 8,
                                  cudaMemcpyDeviceToDevice, b->stream));
     const int len = std::min(K, S - sg * K);
-    FDB_TRY(run_batched(b, len, dt, effective_K(b), effective_shape(b), b->tz, true));
+    FDB_TRY(run_batched(b, len, dt, effective_K(b), effective_shape(b), effective_tz(b), true));
   }
   // lambda_T into the stored layout
   const double* lt = lambda_T;
@@ -1544,10 +1612,12 @@ int fdb_batch_autotune(fdb_batch* b, int num_steps, const double* dt, const char
       std::istringstream ls(line);
       std::string k;
       int K, sh, tz;
-      if (ls >> k >> K >> sh >> tz && k == key && find_variant(K, sh)) {
+      if (ls >> k >> K >> sh >> tz && k == key &&
+          (sh == -1 ? (K >= 2 && K <= 4) : find_variant(K, sh) != nullptr)) {
         b->K = K;
         b->shape = sh;
         b->tz = tz;
+        choose_tuning(b);
         drop_graph(b);
         if (chosen) {
           chosen[0] = K;
@@ -1570,30 +1640,46 @@ int fdb_batch_autotune(fdb_batch* b, int num_steps, const double* dt, const char
     cudaFree(save);
     return fail(FDB_ERR_CUDA, "autotune: cudaEventCreate failed");
   }
+  // {depth, shape, tile_z} as run, and as kept: the automatic choice (its depth,
+  // the rest automatic), then every compiled form that can be asked for, in
+  // whole columns and in ranges of 32 planes
+  struct Try {
+    int K, shape, tz, keep_shape, keep_tz;
+  };
+  const int set[3] = {b->K, b->shape, b->tz};
+  b->K = 0;
+  b->shape = -1;
+  b->tz = 0;
+  choose_tuning(b);
+  std::vector<Try> tries = {{b->eff_K, b->eff_shape, b->eff_tz, -1, 0}};
+  b->K = set[0];
+  b->shape = set[1];
+  b->tz = set[2];
+  choose_tuning(b);
+  const int whole = (int)std::min<uint64_t>(maxn, 1u << 30);
+  for (const Variant& v : kVariants)
+    if (v.shape < fx::kNumShapes)
+      for (int tz : {whole, 32}) tries.push_back({v.K, v.shape, tz, v.shape, tz});
   float best = 1e30f;
-  int bK = kDefaultDepth, bsh = fx::kR4W8S, btz = 0;
+  Try kept = tries[0];
   int rc = FDB_OK;
-  for (const Variant& v : kVariants) {
-    for (int tzc : {0, 32}) {
-      for (int rep = 0; rep < 2 && !rc; ++rep) {  // rep 0 warms up (and builds nothing)
-        b->cur = cur0;
-        cudaMemcpyAsync(b->arena[cur0], save, b->total * 8, cudaMemcpyDeviceToDevice, b->stream);
-        cudaEventRecord(e0, b->stream);
-        rc = run_batched(b, num_steps, dt, v.K, v.shape, tzc, false);
-        cudaEventRecord(e1, b->stream);
-        if (rc == FDB_ERR_UNSUPPORTED) {
-          rc = FDB_OK;
-          break;
-        }
-        if (!rc) rc = bsync(b);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (!rc && rep == 1 && ms < best) {
-          best = ms;
-          bK = v.K;
-          bsh = v.shape;
-          btz = tzc;
-        }
+  for (const Try& t : tries) {
+    for (int rep = 0; rep < 2 && !rc; ++rep) {  // rep 0 warms up (and builds nothing)
+      b->cur = cur0;
+      cudaMemcpyAsync(b->arena[cur0], save, b->total * 8, cudaMemcpyDeviceToDevice, b->stream);
+      cudaEventRecord(e0, b->stream);
+      rc = run_batched(b, num_steps, dt, t.K, t.shape, t.tz, false);
+      cudaEventRecord(e1, b->stream);
+      if (rc == FDB_ERR_UNSUPPORTED) {
+        rc = FDB_OK;
+        break;
+      }
+      if (!rc) rc = bsync(b);
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, e0, e1);
+      if (!rc && rep == 1 && ms < best) {
+        best = ms;
+        kept = t;
       }
     }
   }
@@ -1602,18 +1688,19 @@ int fdb_batch_autotune(fdb_batch* b, int num_steps, const double* dt, const char
   cudaStreamSynchronize(b->stream);
   cudaFree(save);
   if (rc) return rc;
-  b->K = bK;
-  b->shape = bsh;
-  b->tz = btz;
+  b->K = kept.K;
+  b->shape = kept.keep_shape;
+  b->tz = kept.keep_tz;
+  choose_tuning(b);
   drop_graph(b);
   if (chosen) {
-    chosen[0] = bK;
-    chosen[1] = bsh;
-    chosen[2] = btz;
+    chosen[0] = b->K;
+    chosen[1] = b->shape;
+    chosen[2] = b->tz;
   }
   if (cache_path && *cache_path) {
     std::ofstream o(cache_path, std::ios::app);
-    o << key << ' ' << bK << ' ' << bsh << ' ' << btz << '\n';
+    o << key << ' ' << b->K << ' ' << b->shape << ' ' << b->tz << '\n';
   }
   return FDB_OK;
 }
