@@ -846,10 +846,7 @@ int run_looped(fdb_batch* b, int steps, const double* dt, int K) {
       FDB_TRY(launch_advect_fixed_ex(g, c, steps, t, bufs, &cur, b->d_plain_scratch + i * per,
                                      per * 8, nullptr, b->stream));
     } else {
-      for (int s = 0; s < steps; ++s) {
-        FDB_TRY(launch_step_f64(g, c, FDB_ARITH_FMA, bufs[cur], bufs[cur ^ 1], b->stream));
-        cur ^= 1;
-      }
+      FDB_TRY(launch_advect_f64(g, c, FDB_ARITH_FMA, steps, bufs, &cur, b->stream));
     }
     fin[i] = cur;
   }

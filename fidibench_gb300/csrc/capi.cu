@@ -276,11 +276,7 @@ int advance(fdb_upwind* h, int steps, double dt, int arith) {
     return rc;
   }
   h->scale_slot = -1;
-  for (int s = 0; s < steps; ++s) {
-    FDB_TRY(launch_step_f64(g, c, arith, h->buf[h->cur], h->buf[h->cur ^ 1], h->stream));
-    h->cur ^= 1;
-  }
-  return FDB_OK;
+  return launch_advect_f64(g, c, arith, steps, h->buf, &h->cur, h->stream);
 }
 
 // A CUDA event that lives as long as its scope.
@@ -346,11 +342,7 @@ int transposed_steps(fdb_upwind* h, int S, double dt, int arith, int* lc, int* s
                                   h->stream);
   }
   *slot = -1;
-  for (int k = 0; k < S; ++k) {
-    FDB_TRY(launch_step_f64(gT, c, arith, h->lam[*lc], h->lam[*lc ^ 1], h->stream));
-    *lc ^= 1;
-  }
-  return FDB_OK;
+  return launch_advect_f64(gT, c, arith, S, h->lam, lc, h->stream);
 }
 
 // out = (A^T)^S in.  t_done (nullable) is recorded after the last step.

@@ -123,6 +123,10 @@ Coeffs3 coeffs3(const Geom& g, double dt);
 // ---- kernels (launch wrappers return FDB_OK or an error code) -------------
 int launch_step_f64(const Geom& g, const Coeffs3& c, int arith, const double* in,
                     double* out, cudaStream_t s);
+// `steps` FP64 steps through the pair buf (flips *cur), several per launch on
+// small grids; the bits of launch_step_f64 repeated.
+int launch_advect_f64(const Geom& g, const Coeffs3& c, int arith, int steps, double** buf, int* cur,
+                      cudaStream_t s);
 int launch_step_generic(const Geom& g, double dt, const double* in, double* out,
                         cudaStream_t s);
 
