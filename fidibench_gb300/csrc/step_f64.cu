@@ -296,26 +296,6 @@ F64Plan plan_f64(const Geom& g, int arith, int steps) {
   return best;
 }
 
-// Programmatic dependent launch: the kernel's CTAs start while the last ones of
-// the launch before finish, and wait for its end in
-// cudaGridDependencySynchronize, before their first load.  A chain of short
-// launches takes 1.7 us each, the host's own time, instead of 4.1.
-template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
-                             cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at = {};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
-
 template <int ARITH>
 int launch_steps_tile(const TileArgs& a, const Coeffs3& c, const double* in, double* out,
                       cudaStream_t s) {

@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(256)
 k_absmax_bits(const double* __restrict__ f, uint64_t n, ScaleSlot* __restrict__ slot) {
   __shared__ unsigned long long sh[8];
   unsigned long long m = 0ull;
+  cudaGridDependencySynchronize();
   for (uint64_t i = blockIdx.x * 256ull + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256ull) {
     const unsigned long long b =
         (unsigned long long)__double_as_longlong(__ldg(f + i)) & 0x7FFFFFFFFFFFFFFFull;
@@ -341,7 +342,7 @@ int launch_scale_prepass(const Geom& g, const double* f, double* d_scratch, cuda
   uint64_t blocks = (count + 255) / 256;
   if (blocks > 152 * 8) blocks = 152 * 8;
   if (blocks < 1) blocks = 1;
-  k_absmax_bits<<<(unsigned)blocks, 256, 0, s>>>(f + first, count, slots);
+  FDB_CUDA_TRY(launch_dependent(k_absmax_bits, (unsigned)blocks, 256, 0, s, f + first, count, slots));
   note_launch(2);
   FDB_CUDA_TRY(cudaGetLastError());
   return FDB_OK;
