@@ -273,6 +273,9 @@ Config auto_config(const Geom& g, int K_asked) {
     return std::ceil((double)g.nx / (32 - K)) * std::ceil((double)g.ny / (rows - K));
   };
   constexpr double kHalfWave = 152 * 4 / 2;  // CTAs
+  // planes of 4 GB and more: beyond the 4-warp shapes' 32-bit offsets
+  if ((uint64_t)g.ny * g.nx >= (1ull << 29))
+    return {K_asked > 0 ? K_asked : 3, fx::kR6W8L};
   if (tiles(K_hi, 32) * std::ceil(g.nz / 8.0) < kHalfWave) return {K_hi, fx::kR4W4L};
   Config best{K_hi, fx::kR8W4L};
   double best_cost = 0.0;
@@ -294,7 +297,8 @@ Config auto_config(const Geom& g, int K_asked) {
 // 4 rows at 6 CTAs per SM (advect(1) at 256^3, FP64 in and out: 194 GCUPS
 // against 175 for 8 rows).
 int default_shape(const Geom& g, int K, int k) {
-  return k == 1 ? (int)fx::kR4W4L : auto_config(g, K).shape;
+  const int shape = auto_config(g, K).shape;
+  return k == 1 && shape != fx::kR6W8L ? (int)fx::kR4W4L : shape;
 }
 
 }  // namespace

@@ -158,8 +158,12 @@ struct TileGroup {
 // tile_y and Z0 are unused, and every rectangle marches nout + K planes.
 //
 // FULL: the levels whose coefficients in lev have a0 != 0.
+//
+// OFF32: the row offsets are byte offsets in 32 bits (planes below 4 GB), which
+// the memory instructions add to the plane's address themselves; an element
+// offset costs a 64-bit multiply-add per load and store.
 template <int K, int R, int W, bool HSM, int LOADER, int FULL, bool STORE_G = false,
-          bool LEFT_SMEM = false, bool GROUPED = false>
+          bool LEFT_SMEM = false, bool GROUPED = false, bool OFF32 = false>
 __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoeffs& lev, int tile_x, int tile_y, int Z0,
                                              int nout, int levels, bool in_f64, bool out_f64, int s, int d,
                                              const int64_t* __restrict__ in,
@@ -195,7 +199,12 @@ __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoef
     ly = ly < 0 ? ly + a.ny : (ly >= a.ny ? ly - a.ny : ly);  // |ly0| < ny: one wrap at most
     if (ly < 0 || ly >= a.ny) ly = wrap_mod(ly, a.ny);         // grids shorter than the tile
     roff[r] = (a.fy ? a.ny - 1 - ly : ly) * a.nx + px;
+    if (OFF32) roff[r] *= 8u;
   }
+  auto at = [&](auto* plane, int r) {
+    using P = decltype(plane);
+    return OFF32 ? (P)((const char*)plane + roff[r]) : plane + roff[r];
+  };
   // physical offset of the plane at logical z, advanced plane by plane
   const int64_t plane_sz = (int64_t)a.ny * a.nx;
   const int64_t dz = a.fz ? -plane_sz : plane_sz;
@@ -214,6 +223,7 @@ __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoef
   int64_t cur[R];
   static_assert(!LEFT_SMEM || HSM, "the x-1 neighbour from shared memory needs the history there");
   static_assert(!(GROUPED && STORE_G), "packed tiles store no adjoint states");
+  static_assert(!(OFF32 && (STORE_G || LOADER == kLoadCpAsync)), "element offsets there");
   int64_t pre[LOADER != kLoadCpAsync ? R : 1];
 #pragma unroll
   for (int t = 0; t < (HSM ? 1 : K); ++t)
@@ -238,7 +248,7 @@ __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoef
     } else {
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        pre[r] = LOADER == kLoadRegs ? __ldg(src + roff[r]) : __ldcg(src + roff[r]);
+        pre[r] = LOADER == kLoadRegs ? __ldg(at(src, r)) : __ldcg(at(src, r));
     }
   }
 
@@ -264,7 +274,7 @@ __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoef
         const int64_t* src = in + po_next;
 #pragma unroll
         for (int r = 0; r < R; ++r)
-          pre[r] = LOADER == kLoadRegs ? __ldg(src + roff[r]) : __ldcg(src + roff[r]);
+          pre[r] = LOADER == kLoadRegs ? __ldg(at(src, r)) : __ldcg(at(src, r));
       }
     }
     if (in_f64) {
@@ -343,10 +353,7 @@ __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoef
         if (row_mask & (1u << r)) {
           const int64_t v = cur[r];
           if (counted) my_or |= (unsigned long long)(v ^ (v >> 63));
-          if (out_f64)
-            dst[roff[r]] = __double_as_longlong(to_double(v, s));
-          else
-            dst[roff[r]] = v;
+          *at(dst, r) = out_f64 ? __double_as_longlong(to_double(v, s)) : v;
         }
       }
     }
@@ -381,7 +388,7 @@ __device__ __forceinline__ void cta_or(unsigned long long my_or, unsigned long l
 // grid so that the last wave is short (the scheduler hands out CTAs in
 // index order).
 template <int K, int R, int W, bool HSM, int MINB, bool IN_F64, bool OUT_F64, bool STORE_G = false,
-          int LOAD = kLoadCpAsync, bool LEFT = false>
+          int LOAD = kLoadCpAsync, bool LEFT = false, bool OFF32 = false>
 __global__ void __launch_bounds__(32 * W, MINB)
 k_advect_fixed(const int64_t* __restrict__ in, int64_t* __restrict__ out, const FixedArgs a) {
   extern __shared__ __align__(16) int64_t s_dyn[];
@@ -419,7 +426,7 @@ k_advect_fixed(const int64_t* __restrict__ in, int64_t* __restrict__ out, const 
   // the last level of an advect's last launch (the one that writes FP64), and
   // every level of the adjoint's recompute, take 62-bit coefficients
   constexpr int kFull = STORE_G ? kAllFull : (OUT_F64 ? kLastFull : kNoneFull);
-  advance_tile<K, R, W, HSM, LOAD, kFull, STORE_G, LEFT>(a, a.lev, tile % a.tiles_x,
+  advance_tile<K, R, W, HSM, LOAD, kFull, STORE_G, LEFT, false, OFF32>(a, a.lev, tile % a.tiles_x,
                                                          tile / a.tiles_x, z0, nout, K, IN_F64,
                                                          OUT_F64, s, d, in, out, s_dyn, s_row,
                                                          my_or);
@@ -455,11 +462,17 @@ constexpr int shape_warps(int sh) {
 // a.nslab / a.slab_z; returns the CTA count.
 long long plan_slabs(FixedArgs& a, int resident, int cap);
 
+// 32-bit byte offsets for the shapes of the automatic choice at K <= 3, where
+// they measured faster (512^3, 8 x 4, GCUPS: K = 2 553 -> 580, K = 3 617 -> 636,
+// K = 4 583 -> 575).
+constexpr bool use_off32(int K, int W, int load) { return W == 4 && load == kLoadRegs && K <= 3; }
+
 template <int K, int R, int W, bool HSM, int MINB, bool IN, bool OUT, bool STORE_G = false,
           int LOAD = kLoadCpAsync, bool LEFT = false>
 void launch_k(int cap, const int64_t* in, int64_t* out, FixedArgs a, cudaStream_t st) {
   constexpr int smem = fixed_smem_bytes<K, R, W, HSM, LOAD>();
-  auto kern = k_advect_fixed<K, R, W, HSM, MINB, IN, OUT, STORE_G, LOAD, LEFT>;
+  auto kern =
+      k_advect_fixed<K, R, W, HSM, MINB, IN, OUT, STORE_G, LOAD, LEFT, use_off32(K, W, LOAD)>;
   static int per_sm = -1;  // per instantiation; benign race (idempotent)
   if (per_sm < 0) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
