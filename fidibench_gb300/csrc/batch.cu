@@ -93,8 +93,9 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 // spills); 6-row shapes: 20 warps, 8-row shapes: 16 warps (their rows need the
 // registers).  kLeft: the x - 1 neighbour from the plane history (LEFT_SMEM of
 // advance_tile), which the 4-warp shapes take and the 64-register ones do not
-// (slower there).
-template <int K, int R, int W, bool kLeft>
+// (slower there).  kOff32: 32-bit byte offsets (planes below 4 GB), faster at
+// K = 2 (256 uneven instances 447 -> 458 GCUPS) and slower at K = 3.
+template <int K, int R, int W, bool kLeft, bool kOff32>
 __global__ void __launch_bounds__(32 * W, (R > 6 ? 512 : R > 4 ? 640 : 1024) / (32 * W))
 k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ items,
               const fx::TileGroup* __restrict__ groups, int items_per_block, int nblocks,
@@ -181,7 +182,8 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
     // 62 bits; the same code for every block would cost the others the three
     // products and the registers of a0
     auto tile = [&](auto full, int levels, bool out_f64) {
-      fx::advance_tile<K, R, W, true, fx::kLoadL2Regs, decltype(full)::value, false, kLeft, true>(
+      fx::advance_tile<K, R, W, true, fx::kLoadL2Regs, decltype(full)::value, false, kLeft, true,
+                       kOff32>(
           s_a, s_lev, 0, 0, 0, it.nout, levels, b == 0, out_f64, s, d, in, out, s_dyn, s_row,
           my_or, grp, lane - col * it.gw, (warp - rg * it.gh) * R);
     };
@@ -496,7 +498,7 @@ std::array<int, 3> choose_order(const uint64_t n[3]) {
   return best;
 }
 
-template <int K, int R, int W, bool kLeft = false>
+template <int K, int R, int W, bool kLeft = false, bool kOff32 = K == 2>
 int launch_batch_kernel(int grid, const InstDev* insts, const ItemDev* items,
                         const fx::TileGroup* groups, int ipb, int nblocks, int steps, int64_t* a0,
                         int64_t* a1, ScaleSlot* slots, unsigned* done, unsigned* queue, int* err,
@@ -504,22 +506,22 @@ int launch_batch_kernel(int grid, const InstDev* insts, const ItemDev* items,
   constexpr int smem = K * R * 32 * W * (int)sizeof(int64_t);
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(k_batch_fixed<K, R, W, kLeft>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_batch_fixed<K, R, W, kLeft, kOff32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          smem);
     configured = true;
   }
-  k_batch_fixed<K, R, W, kLeft><<<grid, 32 * W, smem, st>>>(insts, items, groups, ipb, nblocks, steps,
+  k_batch_fixed<K, R, W, kLeft, kOff32><<<grid, 32 * W, smem, st>>>(insts, items, groups, ipb, nblocks, steps,
                                                      a0, a1, slots, done, queue, err, wait_bias,
                                                      wait_cycles);
   return FDB_OK;
 }
 
-template <int K, int R, int W, bool kLeft = false>
+template <int K, int R, int W, bool kLeft = false, bool kOff32 = K == 2>
 int resident_ctas_of() {
   constexpr int smem = K * R * 32 * W * (int)sizeof(int64_t);
-  cudaFuncSetAttribute(k_batch_fixed<K, R, W, kLeft>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_batch_fixed<K, R, W, kLeft, kOff32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_fixed<K, R, W, kLeft>, 32 * W, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_fixed<K, R, W, kLeft, kOff32>, 32 * W, smem);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -536,6 +538,7 @@ struct Variant {
   int K, shape;
   LaunchFn launch;
   ResidentFn resident;
+  bool wide = false;  // serves planes of 4 GB and more where another entry does not
 };
 
 // compiled (K, shape) combinations of the batched kernel
@@ -552,11 +555,20 @@ const Variant kVariants[] = {
     // by the automatic choice only
     {2, fx::kR6W4L, launch_batch_kernel<2, 6, 4, true>, resident_ctas_of<2, 6, 4, true>},
     {3, fx::kR6W4L, launch_batch_kernel<3, 6, 4, true>, resident_ctas_of<3, 6, 4, true>},
+    // planes of 4 GB and more at K = 2
+    {2, fx::kR4W16S, launch_batch_kernel<2, 4, 16, false, false>,
+     resident_ctas_of<2, 4, 16, false, false>, true},
+    {2, fx::kR4W8S, launch_batch_kernel<2, 4, 8, false, false>,
+     resident_ctas_of<2, 4, 8, false, false>, true},
+    {2, fx::kR8W8S, launch_batch_kernel<2, 8, 8, false, false>,
+     resident_ctas_of<2, 8, 8, false, false>, true},
+    {2, fx::kR6W4L, launch_batch_kernel<2, 6, 4, true, false>,
+     resident_ctas_of<2, 6, 4, true, false>, true},
 };
 
-const Variant* find_variant(int K, int shape) {
+const Variant* find_variant(int K, int shape, bool wide) {
   for (const Variant& v : kVariants)
-    if (v.K == K && v.shape == shape) return &v;
+    if (v.K == K && v.shape == shape && v.wide == (wide && K == 2)) return &v;
   return nullptr;
 }
 
@@ -669,6 +681,13 @@ int check_dts(fdb_batch* b, const double* dt) {
   return FDB_OK;
 }
 
+// An instance whose plane takes 4 GB or more (beyond 32-bit byte offsets).
+bool wide_planes(const fdb_batch* b) {
+  for (const Geom& g : b->geoms)
+    if ((uint64_t)g.ny * g.nx >= (1ull << 29)) return true;
+  return false;
+}
+
 struct Plan {
   int K, shape, tz;
   const Variant* v;
@@ -684,7 +703,7 @@ int make_plan(fdb_batch* b, int steps, const double* dt, int K, int shape, int t
   p->K = K;
   p->shape = shape;
   p->tz = tz;
-  p->v = find_variant(K, shape);
+  p->v = find_variant(K, shape, wide_planes(b));
   if (!p->v) return fail(FDB_ERR_UNSUPPORTED, "no batched kernel compiled for this depth/shape");
   p->insts.resize(b->count);
   p->items.clear();
@@ -900,7 +919,7 @@ void choose_tuning(fdb_batch* b) {
   for (const Cand& c : list) {
     int tz = b->tz;
     if (tz <= 0) {
-      const Variant* v = find_variant(c.K, c.shape);
+      const Variant* v = find_variant(c.K, c.shape, wide_planes(b));
       pack(c, 0, &items);
       double planes = 0.0;
       for (const ItemDev& it : items) planes += it.nout;
@@ -1610,7 +1629,7 @@ int fdb_batch_autotune(fdb_batch* b, int num_steps, const double* dt, const char
       std::string k;
       int K, sh, tz;
       if (ls >> k >> K >> sh >> tz && k == key &&
-          (sh == -1 ? (K >= 2 && K <= 4) : find_variant(K, sh) != nullptr)) {
+          (sh == -1 ? (K >= 2 && K <= 4) : find_variant(K, sh, false) != nullptr)) {
         b->K = K;
         b->shape = sh;
         b->tz = tz;
@@ -1655,7 +1674,7 @@ int fdb_batch_autotune(fdb_batch* b, int num_steps, const double* dt, const char
   choose_tuning(b);
   const int whole = (int)std::min<uint64_t>(maxn, 1u << 30);
   for (const Variant& v : kVariants)
-    if (v.shape < fx::kNumShapes)
+    if (v.shape < fx::kNumShapes && !v.wide)
       for (int tz : {whole, 32}) tries.push_back({v.K, v.shape, tz, v.shape, tz});
   float best = 1e30f;
   Try kept = tries[0];
