@@ -34,9 +34,10 @@
 // published.  Each instance has its own three-slot scale ring (see
 // step_fixed.cu), advanced per block by the instance's tile 0.
 //
-// The launch sequence of an advect (counter resets, per-instance max|f|
-// pre-pass, persistent kernel) is captured once in a CUDA graph per
-// (steps, dt, tuning) and replayed.
+// An advect is three launches (counter and scale-ring reset, per-instance max|f|
+// pre-pass, persistent kernel), each dependent on the one before.  The device
+// tables of the plan stay until the tuning, a time step or a velocity changes;
+// the forward and the transposed problem have their own.
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -102,6 +103,7 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
               int steps, int64_t* arena0, int64_t* arena1, ScaleSlot* slots, unsigned* done,
               unsigned* queue, int* err, unsigned wait_bias, long long wait_cycles) {
   extern __shared__ __align__(16) int64_t s_dyn[];  // plane history [K][R][threads]
+  cudaGridDependencySynchronize();
   __shared__ int64_t s_row[2][W][32];
   __shared__ unsigned long long s_or[W];
   __shared__ int s_w;
@@ -198,23 +200,34 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
   }
 }
 
-// max|f| of every instance (FP64 bit patterns) into slot 0 of its ring, kind 0;
-// slots 1 and 2 are cleared.  Block b works on instance b / per_inst.
+// max|f| of every instance (FP64 bit patterns) into slot 0 of its ring (kind 0,
+// cleared by k_batch_reset).  Block b works on instance b / per_inst; four loads
+// in flight per thread.
 __global__ void __launch_bounds__(256)
-k_batch_absmax(const double* __restrict__ arena, const InstDev* __restrict__ insts, int count,
-               int per_inst, ScaleSlot* slots) {
+k_batch_absmax(const double* __restrict__ arena, const int64_t* __restrict__ offs,
+               const uint64_t* __restrict__ sizes, int per_inst, ScaleSlot* slots) {
   __shared__ unsigned long long sh[8];
   const int i = blockIdx.x / per_inst;
   const int part = blockIdx.x - i * per_inst;
-  if (i >= count) return;
-  const InstDev& I = insts[i];
-  const uint64_t n = (uint64_t)I.a.nx * I.a.ny * I.a.nz;
+  const double* f = arena + offs[i];
+  const uint64_t n = sizes[i];
+  const uint64_t step = (uint64_t)per_inst * 256;
+  cudaGridDependencySynchronize();
   unsigned long long m = 0ull;
-  for (uint64_t k = (uint64_t)part * 256 + threadIdx.x; k < n; k += (uint64_t)per_inst * 256) {
+  auto take = [&](double x) {
     const unsigned long long bits =
-        (unsigned long long)__double_as_longlong(__ldg(arena + I.offset + k)) & 0x7FFFFFFFFFFFFFFFull;
+        (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
     m = bits > m ? bits : m;
+  };
+  uint64_t k = (uint64_t)part * 256 + threadIdx.x;
+  for (; k + 3 * step < n; k += 4 * step) {
+    const double x0 = f[k], x1 = f[k + step], x2 = f[k + 2 * step], x3 = f[k + 3 * step];
+    take(x0);
+    take(x1);
+    take(x2);
+    take(x3);
   }
+  for (; k < n; k += step) take(f[k]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
@@ -228,11 +241,14 @@ k_batch_absmax(const double* __restrict__ arena, const InstDev* __restrict__ ins
   }
 }
 
-__global__ void k_batch_slots_init(ScaleSlot* slots, int count) {
+// Work queue, completion counters and scale rings at the start of an advect.
+__global__ void k_batch_reset(ScaleSlot* slots, unsigned* done, unsigned* queue, int count) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 3 * count; k += gridDim.x * blockDim.x) {
     slots[k].m = 0ull;
     slots[k].s = 0;
     slots[k].kind = (k % 3 == 0) ? 0 : 1;
+    if (k < count) done[k] = 0u;
+    if (k == 0) *queue = 0u;
   }
 }
 
@@ -510,9 +526,9 @@ int launch_batch_kernel(int grid, const InstDev* insts, const ItemDev* items,
                          smem);
     configured = true;
   }
-  k_batch_fixed<K, R, W, kLeft, kOff32><<<grid, 32 * W, smem, st>>>(insts, items, groups, ipb, nblocks, steps,
-                                                     a0, a1, slots, done, queue, err, wait_bias,
-                                                     wait_cycles);
+  FDB_CUDA_TRY(launch_dependent(k_batch_fixed<K, R, W, kLeft, kOff32>, (unsigned)grid, 32 * W, smem,
+                                st, insts, items, groups, ipb, nblocks, steps, a0, a1, slots,
+                                done, queue, err, wait_bias, wait_cycles));
   return FDB_OK;
 }
 
@@ -578,6 +594,19 @@ const Variant* find_variant(int K, int shape, bool wide) {
 using namespace fdb;
 using namespace fdb::bt;
 
+// A plan and its device tables.
+struct PlanTables {
+  const Variant* v = nullptr;  // null: no plan
+  int shape = -1, tz = 0;
+  std::vector<double> dt;
+  int ipb = 0, resident = 0;
+  InstDev* d_insts = nullptr;
+  ItemDev* d_items = nullptr;
+  size_t item_cap = 0;
+  fx::TileGroup* d_groups = nullptr;
+  size_t group_cap = 0;
+};
+
 struct fdb_batch {
   int count = 0;
   std::vector<Geom> geoms;      // as stored (the kernels' geometry)
@@ -596,9 +625,6 @@ struct fdb_batch {
   double* adj_dda = nullptr;
   void* adj_scratch = nullptr;
   size_t adj_scratch_bytes = 0;
-  // plans built while set step the transposed problem (every upwind
-  // direction reversed, the coefficients unchanged): the dL/df0-only adjoint
-  bool transposed_run = false;
   // adjoint form (FDB_TUNE_ADJOINT): 0 = dL/dv in closed form, 1 = step by step
   int adj_mode = 0;
   DeviceScratch contract;  // the closed form's contraction tables and partials
@@ -607,12 +633,7 @@ struct fdb_batch {
   int64_t total = 0;
   double* arena[2] = {nullptr, nullptr};
   int cur = 0;
-  // device tables
-  InstDev* d_insts = nullptr;
-  ItemDev* d_items = nullptr;
-  size_t item_cap = 0;
-  fx::TileGroup* d_groups = nullptr;
-  size_t group_cap = 0;
+  PlanTables tables[2];  // the forward problem's, the transposed one's
   ScaleSlot* d_slots = nullptr;
   unsigned* d_done = nullptr;
   unsigned* d_queue = nullptr;
@@ -629,9 +650,6 @@ struct fdb_batch {
   // tuning as set (0 / -1 = automatic), and what the launches take
   int K = 0, shape = -1, tz = 0;
   int eff_K = 0, eff_shape = -1, eff_tz = 0;
-  // graph cache
-  cudaGraphExec_t graph = nullptr;
-  std::string graph_key;
 };
 
 namespace {
@@ -644,9 +662,10 @@ int bcheck(fdb_batch* b) {
 }
 
 int bsync(fdb_batch* b) {
+  int* h_err = reinterpret_cast<int*>(b->h_sums + b->count);
+  FDB_CUDA_TRY(cudaMemcpyAsync(h_err, b->d_err, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
   FDB_CUDA_TRY(cudaStreamSynchronize(b->stream));
-  int herr = 0;
-  FDB_CUDA_TRY(cudaMemcpy(&herr, b->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  const int herr = *h_err;
   if (herr) {
     FDB_CUDA_TRY(cudaMemset(b->d_err, 0, sizeof(int)));
     if (herr & 2)
@@ -668,10 +687,9 @@ int balloc(T** p, size_t count) {
   return FDB_OK;
 }
 
-void drop_graph(fdb_batch* b) {
-  if (b->graph) cudaGraphExecDestroy(b->graph);
-  b->graph = nullptr;
-  b->graph_key.clear();
+// The tuning or a velocity changed: the plans are built again.
+void drop_plans(fdb_batch* b) {
+  for (PlanTables& t : b->tables) t.v = nullptr;
 }
 
 int check_dts(fdb_batch* b, const double* dt) {
@@ -688,157 +706,106 @@ bool wide_planes(const fdb_batch* b) {
   return false;
 }
 
-struct Plan {
-  int K, shape, tz;
-  const Variant* v;
-  std::vector<InstDev> insts;
+// The plan of an advect with these settings into `t` (kept from the last call if
+// nothing changed): tiles, instance arguments, their device copies.  transposed:
+// every upwind direction reversed, the coefficients unchanged.
+int make_plan(fdb_batch* b, const double* dt, int K, int shape, int tz, bool transposed,
+              PlanTables* t) {
+  if (t->v && t->v->K == K && t->shape == shape && t->tz == tz &&
+      memcmp(t->dt.data(), dt, b->count * sizeof(double)) == 0)
+    return FDB_OK;
+  t->v = nullptr;
+  const Variant* v = find_variant(K, shape, wide_planes(b));
+  if (!v) return fail(FDB_ERR_UNSUPPORTED, "no batched kernel compiled for this depth/shape");
+  std::vector<InstDev> insts(b->count);
   std::vector<ItemDev> items;
   std::vector<fx::TileGroup> groups;
-  int ipb = 0;
-  int nblocks = 0;
-  int grid = 0;
-};
-
-int make_plan(fdb_batch* b, int steps, const double* dt, int K, int shape, int tz, Plan* p) {
-  p->K = K;
-  p->shape = shape;
-  p->tz = tz;
-  p->v = find_variant(K, shape, wide_planes(b));
-  if (!p->v) return fail(FDB_ERR_UNSUPPORTED, "no batched kernel compiled for this depth/shape");
-  p->insts.resize(b->count);
-  p->items.clear();
-  p->groups.clear();
-  const int resident = p->v->resident();
+  const int resident = v->resident();
   const int R = fx::shape_rows(shape), W = fx::shape_warps(shape);
   int base = 0;
   for (int i = 0; i < b->count; ++i) {
     const Geom& g = b->geoms[i];
     const Coeffs3 c = coeffs3(g, dt[i]);
     if (fixed_supported(g, c, K) != FDB_OK) return FDB_ERR_UNSUPPORTED;
-    InstDev& I = p->insts[i];
-    // per instance: whole z extent per tile unless tz is given (many small
-    // instances already fill the device)
-    I.a = make_fixed_args(b->transposed_run ? transposed_geom(g) : g, c, shape, K,
+    InstDev& I = insts[i];
+    I.a = make_fixed_args(transposed ? transposed_geom(g) : g, c, shape, K,
                           tz > 0 ? tz : (int)g.nz, resident);
     I.a.scale_log = nullptr;
     I.offset = b->offsets[i];
-    const size_t first = p->items.size();
-    FDB_TRY(pack_instance(I.a.nx, I.a.ny, I.a.nz, i, K, R, W, tz, &p->items, &p->groups));
-    const size_t items = p->items.size() - first;
-    if (items > (1u << 24)) return fail(FDB_ERR_UNSUPPORTED, "instance has too many tiles");
-    I.items = (int)items;
+    const size_t first = items.size();
+    FDB_TRY(pack_instance(I.a.nx, I.a.ny, I.a.nz, i, K, R, W, tz, &items, &groups));
+    const size_t n = items.size() - first;
+    if (n > (1u << 24)) return fail(FDB_ERR_UNSUPPORTED, "instance has too many tiles");
+    I.items = (int)n;
     I.item_base = base;
     base += I.items;
   }
-  if (p->groups.size() >= (1ull << 31))
+  if (groups.size() >= (1ull << 31))
     return fail(FDB_ERR_UNSUPPORTED, "batched plan exceeds 2^31 tile rectangles");
-  p->ipb = base;
-  p->nblocks = (steps + K - 1) / K;
-  if ((int64_t)p->nblocks * p->ipb >= (1ll << 31))
-    return fail(FDB_ERR_UNSUPPORTED, "batched work queue exceeds 2^31 items");
-  p->grid = (int)std::min<int64_t>((int64_t)p->nblocks * p->ipb, resident);
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  FDB_CUDA_TRY(cudaStreamIsCapturing(b->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone)
+    return fail(FDB_ERR_CUDA, "a batched advect with new settings cannot be captured (its tables "
+                              "are copied from the host): run it once before the capture");
+  if (!t->d_insts) FDB_TRY(balloc(&t->d_insts, (size_t)b->count));
+  if (items.size() > t->item_cap) {
+    if (t->d_items) cudaFree(t->d_items);
+    t->d_items = nullptr;
+    t->item_cap = 0;
+    FDB_TRY(balloc(&t->d_items, items.size()));
+    t->item_cap = items.size();
+  }
+  if (groups.size() > t->group_cap) {
+    if (t->d_groups) cudaFree(t->d_groups);
+    t->d_groups = nullptr;
+    t->group_cap = 0;
+    FDB_TRY(balloc(&t->d_groups, groups.size()));
+    t->group_cap = groups.size();
+  }
+  // pageable sources: the copies are staged before cudaMemcpyAsync returns
+  FDB_CUDA_TRY(cudaMemcpyAsync(t->d_insts, insts.data(), insts.size() * sizeof(InstDev),
+                               cudaMemcpyHostToDevice, b->stream));
+  FDB_CUDA_TRY(cudaMemcpyAsync(t->d_items, items.data(), items.size() * sizeof(ItemDev),
+                               cudaMemcpyHostToDevice, b->stream));
+  FDB_CUDA_TRY(cudaMemcpyAsync(t->d_groups, groups.data(), groups.size() * sizeof(fx::TileGroup),
+                               cudaMemcpyHostToDevice, b->stream));
+  t->shape = shape;
+  t->tz = tz;
+  t->dt.assign(dt, dt + b->count);
+  t->ipb = base;
+  t->resident = resident;
+  t->v = v;
   return FDB_OK;
 }
 
-// Enqueue one batched advect (not captured).
-int enqueue_advect(fdb_batch* b, const Plan& p, int steps, cudaStream_t st) {
-  FDB_CUDA_TRY(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned), st));
-  FDB_CUDA_TRY(cudaMemsetAsync(b->d_done, 0, b->count * sizeof(unsigned), st));
-  k_batch_slots_init<<<(3 * b->count + 255) / 256, 256, 0, st>>>(b->d_slots, b->count);
-  const int per_inst = 8;
-  k_batch_absmax<<<b->count * per_inst, 256, 0, st>>>(b->arena[b->cur], b->d_insts, b->count,
-                                                       per_inst, b->d_slots);
+int run_batched(fdb_batch* b, int steps, const double* dt, int K, int shape, int tz,
+                bool transposed = false) {
+  PlanTables& t = b->tables[transposed ? 1 : 0];
+  FDB_TRY(make_plan(b, dt, K, shape, tz, transposed, &t));
+  const int nblocks = (steps + K - 1) / K;
+  if ((int64_t)nblocks * t.ipb >= (1ll << 31))
+    return fail(FDB_ERR_UNSUPPORTED, "batched work queue exceeds 2^31 items");
+  const int grid = (int)std::min<int64_t>((int64_t)nblocks * t.ipb, t.resident);
+  cudaStream_t st = b->stream;
+  k_batch_reset<<<(3 * b->count + 255) / 256, 256, 0, st>>>(b->d_slots, b->d_done, b->d_queue,
+                                                            b->count);
+  // a wave of blocks over all instances, and the largest one's share per block short
+  const uint64_t largest = *std::max_element(b->sizes.begin(), b->sizes.end());
+  const int per_inst = (int)std::min<uint64_t>(
+      4096, std::max<uint64_t>({8, (uint64_t)(152 * 8 / b->count), largest / 32768}));
+  FDB_CUDA_TRY(launch_dependent(k_batch_absmax, (unsigned)(b->count * per_inst), 256, 0, st,
+                                b->arena[b->cur], b->d_offs, b->d_sizes, per_inst, b->d_slots));
   int64_t* a0 = (int64_t*)b->arena[b->cur];
   int64_t* a1 = (int64_t*)b->arena[b->cur ^ 1];
   // FDB_FAULT=timeout makes every dependency unsatisfiable and the wait
   // budget ~1 ms, so the bounded-wait error path runs without a GPU fault
   const bool inject = fault_injected("timeout");
-  p.v->launch(p.grid, b->d_insts, b->d_items, b->d_groups, p.ipb, p.nblocks, steps, a0, a1,
-              b->d_slots, b->d_done, b->d_queue, b->d_err, inject ? (1u << 30) : 0u,
-              inject ? 2000000ll : kWaitCycles, st);
+  FDB_TRY(t.v->launch(grid, t.d_insts, t.d_items, t.d_groups, t.ipb, nblocks, steps, a0, a1,
+                      b->d_slots, b->d_done, b->d_queue, b->d_err, inject ? (1u << 30) : 0u,
+                      inject ? 2000000ll : kWaitCycles, st));
   note_launch(3);
   FDB_CUDA_TRY(cudaGetLastError());
-  return FDB_OK;
-}
-
-int upload_plan(fdb_batch* b, const Plan& p) {
-  if (p.items.size() > b->item_cap) {
-    if (b->d_items) cudaFree(b->d_items);
-    b->d_items = nullptr;
-    b->item_cap = 0;
-    FDB_TRY(balloc(&b->d_items, p.items.size()));
-    b->item_cap = p.items.size();
-  }
-  if (p.groups.size() > b->group_cap) {
-    if (b->d_groups) cudaFree(b->d_groups);
-    b->d_groups = nullptr;
-    b->group_cap = 0;
-    FDB_TRY(balloc(&b->d_groups, p.groups.size()));
-    b->group_cap = p.groups.size();
-  }
-  FDB_CUDA_TRY(cudaMemcpyAsync(b->d_insts, p.insts.data(), p.insts.size() * sizeof(InstDev),
-                               cudaMemcpyHostToDevice, b->stream));
-  FDB_CUDA_TRY(cudaMemcpyAsync(b->d_items, p.items.data(), p.items.size() * sizeof(ItemDev),
-                               cudaMemcpyHostToDevice, b->stream));
-  FDB_CUDA_TRY(cudaMemcpyAsync(b->d_groups, p.groups.data(),
-                               p.groups.size() * sizeof(fx::TileGroup), cudaMemcpyHostToDevice,
-                               b->stream));
-  return FDB_OK;
-}
-
-std::string plan_key(fdb_batch* b, int steps, const double* dt, const Plan& p) {
-  std::ostringstream os;
-  os << steps << ':' << p.K << ':' << p.shape << ':' << p.tz << ':' << b->cur << ':'
-     << (void*)b->stream << ':' << b->transposed_run;
-  uint64_t h = 1469598103934665603ull;
-  for (int i = 0; i < b->count; ++i) {
-    uint64_t x;
-    memcpy(&x, &dt[i], 8);
-    h = (h ^ x) * 1099511628211ull;
-  }
-  os << ':' << h;
-  return os.str();
-}
-
-int run_batched(fdb_batch* b, int steps, const double* dt, int K, int shape, int tz,
-                bool use_graph) {
-  Plan p;
-  const int rc = make_plan(b, steps, dt, K, shape, tz, &p);
-  if (rc) return rc;
-  const std::string key = plan_key(b, steps, dt, p);
-  if (fault_injected("timeout")) use_graph = false;
-  if (use_graph && b->graph && key == b->graph_key) {
-    FDB_CUDA_TRY(cudaGraphLaunch(b->graph, b->stream));
-    note_launch(3);
-  } else {
-    FDB_TRY(upload_plan(b, p));
-    if (use_graph) {
-      drop_graph(b);
-      cudaStream_t cs = nullptr;
-      FDB_CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-      // the plan upload above is ordered before the capture stream's work
-      cudaStreamSynchronize(b->stream);
-      cudaGraph_t graph = nullptr;
-      cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-      int rc2 = FDB_OK;
-      if (e == cudaSuccess) {
-        rc2 = enqueue_advect(b, p, steps, cs);
-        e = cudaStreamEndCapture(cs, &graph);
-      }
-      if (e == cudaSuccess && rc2 == FDB_OK)
-        e = cudaGraphInstantiate(&b->graph, graph, 0);
-      if (graph) cudaGraphDestroy(graph);
-      cudaStreamDestroy(cs);
-      if (rc2) return rc2;
-      FDB_CUDA_TRY(e);
-      b->graph_key = key;
-      FDB_CUDA_TRY(cudaGraphLaunch(b->graph, b->stream));
-    } else {
-      drop_graph(b);  // the device tables now hold this plan, not the cached graph's
-      FDB_TRY(enqueue_advect(b, p, steps, b->stream));
-    }
-  }
-  b->cur ^= (p.nblocks & 1);
+  b->cur ^= (nblocks & 1);
   return FDB_OK;
 }
 
@@ -1118,7 +1085,7 @@ int fdb_batch_create(int count, const fdb_instance_desc* descs, fdb_batch** out)
   const size_t per = (fixed_scratch_bytes() + 7) / 8;
   int rc = FDB_OK;
   if ((rc = balloc(&b->arena[0], b->total)) || (rc = balloc(&b->arena[1], b->total)) ||
-      (rc = balloc(&b->d_insts, count)) || (rc = balloc(&b->d_slots, 3 * count)) ||
+      (rc = balloc(&b->d_slots, 3 * count)) ||
       (rc = balloc(&b->d_done, count)) || (rc = balloc(&b->d_queue, 1)) ||
       (rc = balloc(&b->d_err, 1)) || (rc = balloc(&b->d_offs, count)) ||
       (rc = balloc(&b->d_sizes, count)) || (rc = balloc(&b->d_part, count * kSumPerInst)) ||
@@ -1127,7 +1094,7 @@ int fdb_batch_create(int count, const fdb_instance_desc* descs, fdb_batch** out)
     fdb_batch_destroy(b);
     return rc;
   }
-  e = cudaMallocHost((void**)&b->h_sums, count * sizeof(double));
+  e = cudaMallocHost((void**)&b->h_sums, (count + 1) * sizeof(double));  // and the error word
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_plain_scratch, 0, per * count * 8, b->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->arena[0], 0, b->total * 8, b->stream);
@@ -1156,13 +1123,17 @@ int fdb_batch_create(int count, const fdb_instance_desc* descs, fdb_batch** out)
 int fdb_batch_destroy(fdb_batch* b) {
   if (!b) return FDB_OK;
   if (b->stream) cudaStreamSynchronize(b->stream);
-  drop_graph(b);
-  void* ps[] = {b->arena[0], b->arena[1], b->d_insts, b->d_items,  b->d_groups,
-                b->d_slots,  b->d_done,  b->d_queue, b->d_err,    b->d_offs,
+  drop_plans(b);
+  void* ps[] = {b->arena[0], b->arena[1], b->d_slots,  b->d_done,  b->d_queue, b->d_err,    b->d_offs,
                 b->d_sizes,  b->d_part,  b->d_sums,  b->d_plain_scratch, b->d_stage,
                 b->d_io};
   for (void* p : ps)
     if (p) cudaFree(p);
+  for (PlanTables& t : b->tables) {
+    cudaFree(t.d_insts);
+    cudaFree(t.d_items);
+    cudaFree(t.d_groups);
+  }
   free_batch_adjoint(b);
   b->contract.release();
   if (b->h_sums) cudaFreeHost(b->h_sums);
@@ -1196,7 +1167,7 @@ int fdb_batch_set_velocity(fdb_batch* b, int index, const double* velocity) {
   FDB_TRY(bsync(b));
   b->geoms_ref[index] = g;
   b->geoms[index] = gs;
-  drop_graph(b);
+  drop_plans(b);
   return FDB_OK;
 }
 
@@ -1284,7 +1255,7 @@ int fdb_batch_set_stream(fdb_batch* b, void* cuda_stream) {
   FDB_TRY(bcheck(b));
   FDB_TRY(bsync(b));
   b->stream = cuda_stream ? (cudaStream_t)cuda_stream : b->own;
-  drop_graph(b);
+  drop_plans(b);
   return FDB_OK;
 }
 
@@ -1308,7 +1279,7 @@ int fdb_batch_set_tuning(fdb_batch* b, int key, int value) {
     return fail(FDB_ERR_INVALID, "unknown tuning key");
   }
   choose_tuning(b);
-  drop_graph(b);
+  drop_plans(b);
   return FDB_OK;
 }
 
@@ -1318,7 +1289,7 @@ int fdb_batch_advect(fdb_batch* b, int num_steps, const double* dt) {
   if (num_steps < 0) return fail(FDB_ERR_INVALID, "num_steps must be >= 0");
   FDB_TRY(check_dts(b, dt));
   if (num_steps == 0) return FDB_OK;
-  const int rc = run_batched(b, num_steps, dt, effective_K(b), effective_shape(b), effective_tz(b), true);
+  const int rc = run_batched(b, num_steps, dt, effective_K(b), effective_shape(b), effective_tz(b));
   if (rc == FDB_ERR_UNSUPPORTED) {
     // some instance is outside the fixed kernel's domain: loop the plain path
     return run_looped(b, num_steps, dt, effective_K(b));
@@ -1368,13 +1339,11 @@ static int batch_lam_steps(fdb_batch* b, int S, const double* dt, int* lc) {
   std::swap(b->arena[0], b->adj_lam[0]);
   std::swap(b->arena[1], b->adj_lam[1]);
   b->cur = *lc;
-  b->transposed_run = true;
-  const int rc = run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b), false);
+  const int rc = run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b), true);
   *lc = b->cur;
   std::swap(b->arena[0], b->adj_lam[0]);
   std::swap(b->arena[1], b->adj_lam[1]);
   b->cur = cur;
-  b->transposed_run = false;
   return rc;
 }
 
@@ -1431,7 +1400,7 @@ static int batch_adjoint_closed_form(fdb_batch* b, int S, const double* dt,
   FDB_TRY(batch_lam_steps(b, 1, dt, &lc));
   FDB_TRY(batch_lam_store(b, lc, grad_f0, is_device));
   if (advance_fields)
-    FDB_TRY(run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b), true));
+    FDB_TRY(run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b)));
   std::vector<double> dda(3 * (size_t)n);
   FDB_CUDA_TRY(cudaMemcpyAsync(dda.data(), b->adj_dda, dda.size() * 8, cudaMemcpyDeviceToHost,
                                b->stream));
@@ -1446,7 +1415,7 @@ static int batch_adjoint_closed_form(fdb_batch* b, int S, const double* dt,
 static int batch_adjoint_f0_only(fdb_batch* b, int S, const double* dt, const double* lambda_T,
                                  double* grad_f0, int is_device) {
   if (S > 0 && b->adj_mode != 2)  // form 2 keeps the fields at f0
-    FDB_TRY(run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b), true));
+    FDB_TRY(run_batched(b, S, dt, effective_K(b), effective_shape(b), effective_tz(b)));
   return batch_transposed(b, S, dt, lambda_T, grad_f0, is_device);
 }
 
@@ -1532,7 +1501,7 @@ int fdb_batch_adjoint(fdb_batch* b, int num_steps, const double* dt, const doubl
     FDB_CUDA_TRY(cudaMemcpyAsync(b->adj_ckpt[sg], b->arena[b->cur], T * 8,
                                  cudaMemcpyDeviceToDevice, b->stream));
     const int len = std::min(K, S - sg * K);
-    FDB_TRY(run_batched(b, len, dt, effective_K(b), effective_shape(b), effective_tz(b), true));
+    FDB_TRY(run_batched(b, len, dt, effective_K(b), effective_shape(b), effective_tz(b)));
   }
   // lambda_T into the stored layout
   const double* lt = lambda_T;
@@ -1634,7 +1603,7 @@ int fdb_batch_autotune(fdb_batch* b, int num_steps, const double* dt, const char
         b->shape = sh;
         b->tz = tz;
         choose_tuning(b);
-        drop_graph(b);
+        drop_plans(b);
         if (chosen) {
           chosen[0] = K;
           chosen[1] = sh;
@@ -1684,7 +1653,7 @@ int fdb_batch_autotune(fdb_batch* b, int num_steps, const double* dt, const char
       b->cur = cur0;
       cudaMemcpyAsync(b->arena[cur0], save, b->total * 8, cudaMemcpyDeviceToDevice, b->stream);
       cudaEventRecord(e0, b->stream);
-      rc = run_batched(b, num_steps, dt, t.K, t.shape, t.tz, false);
+      rc = run_batched(b, num_steps, dt, t.K, t.shape, t.tz);
       cudaEventRecord(e1, b->stream);
       if (rc == FDB_ERR_UNSUPPORTED) {
         rc = FDB_OK;
@@ -1708,7 +1677,7 @@ int fdb_batch_autotune(fdb_batch* b, int num_steps, const double* dt, const char
   b->shape = kept.keep_shape;
   b->tz = kept.keep_tz;
   choose_tuning(b);
-  drop_graph(b);
+  drop_plans(b);
   if (chosen) {
     chosen[0] = b->K;
     chosen[1] = b->shape;

@@ -293,8 +293,9 @@ int fdb_upwind_adjoint_step(fdb_upwind* h, double dt, const double* f_dev,
  * uneven sizes and velocities, each one the reference's Upwind<ndims>
  * (upwind.cxx:23-49) with ndims <= 3, advanced together.
  * fdb_batch_advect runs one persistent launch per call (all instances, all
- * time blocks, per-instance dependency tracking with bounded waits; replayed
- * from a CUDA graph when called again with the same steps, dt and tuning).
+ * time blocks, per-instance dependency tracking with bounded waits; its tables
+ * are kept while dt, the velocities and the tuning stay the same, and have to
+ * be there before the call is captured into a CUDA graph).
  * fdb_batch_advect_looped is the comparator: the single-field kernel looped
  * over the instances, with the depth set by FDB_TUNE_DEPTH (equal depths
  * give bit-identical fields) or, without one, each instance's single-field
