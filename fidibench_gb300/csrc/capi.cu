@@ -24,7 +24,8 @@ struct fdb_upwind {
   double* part = nullptr;     // reduction partials (reduce_partials(ntot))
   double* dscal = nullptr;    // device scalars [8]
   double* dpart = nullptr;    // adjoint per-CTA coefficient partials [3 * adjoint_blocks()]
-  double* hscal = nullptr;    // pinned host scalars [8]
+  double* hscal = nullptr;    // pinned host scalars [8], then copies of the two error words
+  bool fixed_ran = false;     // a fixed-point launch was made: the error words can be set
   double* scratch = nullptr;  // fixed-point path: max|f| slots + error word
   size_t scratch_bytes = 0;
   int scale_slot = -1;        // scratch slot holding max|f| of the current field (-1: unknown)
@@ -182,15 +183,12 @@ int check_no_chain(fdb_upwind* h) {
   return FDB_OK;
 }
 
-// Report (and clear) the error word that the fixed-point kernels set in a
-// scratch block when they meet a non-finite input.  The stream must be
-// synchronised.
-int check_error_word(double* scratch, const char* what) {
-  int* err = fixed_error_word(scratch);
-  int herr = 0;
-  FDB_CUDA_TRY(cudaMemcpy(&herr, err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (herr) {
-    FDB_CUDA_TRY(cudaMemset(err, 0, sizeof(int)));
+// Report (and clear) an error word that the fixed-point kernels set in a
+// scratch block when they meet a non-finite input; `word` is its value.  The
+// stream must be synchronised.
+int check_error_word(int word, double* scratch, const char* what) {
+  if (word) {
+    FDB_CUDA_TRY(cudaMemset(fixed_error_word(scratch), 0, sizeof(int)));
     return fail(FDB_ERR_NONFINITE, std::string(what) +
                                        " holds NaN or Inf values (the fixed-point kernel needs "
                                        "finite input)");
@@ -198,11 +196,22 @@ int check_error_word(double* scratch, const char* what) {
   return FDB_OK;
 }
 
-// Synchronise the handle's stream and report a non-finite field.
+// Synchronise the handle's stream and report a non-finite field: the error
+// words are copied behind the stream's work, so that one wait serves both, and
+// only if a fixed-point kernel, which alone sets them, has run.
 int sync(fdb_upwind* h) {
+  int* words = reinterpret_cast<int*>(h->hscal + 8);
+  words[0] = words[1] = 0;
+  if (h->fixed_ran) {
+    FDB_CUDA_TRY(cudaMemcpyAsync(&words[0], fixed_error_word(h->scratch), sizeof(int),
+                                 cudaMemcpyDeviceToHost, h->stream));
+    if (h->tscratch)
+      FDB_CUDA_TRY(cudaMemcpyAsync(&words[1], fixed_error_word(h->tscratch), sizeof(int),
+                                   cudaMemcpyDeviceToHost, h->stream));
+  }
   FDB_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  FDB_TRY(check_error_word(h->scratch, "the field"));
-  if (h->tscratch) FDB_TRY(check_error_word(h->tscratch, "the transposed input"));
+  FDB_TRY(check_error_word(words[0], h->scratch, "the field"));
+  if (h->tscratch) FDB_TRY(check_error_word(words[1], h->tscratch, "the transposed input"));
   return FDB_OK;
 }
 
@@ -270,6 +279,7 @@ int advance(fdb_upwind* h, int steps, double dt, int arith) {
   const Coeffs3 c = coeffs3(g, dt);
   if (arith == FDB_ARITH_FIXED) {
     h->tune.depth = h->depth;
+    h->fixed_ran = true;
     const int rc = launch_advect_fixed_ex(g, c, steps, h->tune, h->buf, &h->cur, h->scratch,
                                           h->scratch_bytes, &h->scale_slot, h->stream);
     if (rc) h->scale_slot = -1;
@@ -338,6 +348,7 @@ int transposed_steps(fdb_upwind* h, int S, double dt, int arith, int* lc, int* s
   if (arith == FDB_ARITH_FIXED) {
     FixedTuning t = h->tune;
     t.depth = h->depth;
+    h->fixed_ran = true;
     return launch_advect_fixed_ex(gT, c, S, t, h->lam, lc, h->tscratch, h->scratch_bytes, slot,
                                   h->stream);
   }
@@ -512,7 +523,7 @@ int create_handle(int ndims, const double* velocity, const double* lengths,
   }
   h->scratch_bytes = (fixed_scratch_bytes() + 7) / 8 * 8;
   e = cudaMemsetAsync(h->scratch, 0, h->scratch_bytes, h->stream);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&h->hscal, 8 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&h->hscal, 9 * sizeof(double));
   if (e != cudaSuccess) {
     fdb_upwind_destroy(h);
     return cuda_fail(e, "cudaMallocHost");
@@ -608,6 +619,7 @@ int fdb_upwind_block_begin(fdb_upwind* h, double dt, int* fixed) {
   h->chain_first = 1;
   h->chain_carry = CoeffCarry();
   if (arith == FDB_ARITH_FIXED) {
+    h->fixed_ran = true;
     h->chain_K = h->depth > 0 ? h->depth : default_depth(h->g);
     if (h->scale_slot < 0) {
       FDB_TRY(launch_scale_prepass(h->g, h->buf[h->cur], h->scratch, h->stream));

@@ -80,11 +80,21 @@ k_absmax_bits(const double* __restrict__ f, uint64_t n, ScaleSlot* __restrict__ 
   __shared__ unsigned long long sh[8];
   unsigned long long m = 0ull;
   cudaGridDependencySynchronize();
-  for (uint64_t i = blockIdx.x * 256ull + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256ull) {
+  auto take = [&](double x) {
     const unsigned long long b =
-        (unsigned long long)__double_as_longlong(__ldg(f + i)) & 0x7FFFFFFFFFFFFFFFull;
+        (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
     m = b > m ? b : m;
+  };
+  const uint64_t step = (uint64_t)gridDim.x * 256ull;
+  uint64_t i = blockIdx.x * 256ull + threadIdx.x;
+  for (; i + 3 * step < n; i += 4 * step) {  // four loads in flight
+    const double x0 = f[i], x1 = f[i + step], x2 = f[i + 2 * step], x3 = f[i + 3 * step];
+    take(x0);
+    take(x1);
+    take(x2);
+    take(x3);
   }
+  for (; i < n; i += step) take(f[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);

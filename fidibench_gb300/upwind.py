@@ -188,7 +188,10 @@ class Upwind:
     def set_field(self, values) -> None:
         """setInitialCondition: numpy array (host) or CUDA torch tensor (device)."""
         if hasattr(values, "is_cuda") and values.is_cuda:
-            t = values.detach().to(dtype=__import__("torch").float64).contiguous()
+            import torch
+            t = values
+            if t.dtype != torch.float64 or not t.is_contiguous():
+                t = t.detach().to(dtype=torch.float64).contiguous()
             if t.numel() != self.ntot:
                 raise ValueError(f"field has {t.numel()} values, expected {self.ntot}")
             _order_after_torch(t)
