@@ -166,22 +166,29 @@ fx::FixedArgs make_fixed_args(const Geom& g, const Coeffs3& c, int shape, int K,
 
 namespace fx {
 
-long long plan_slabs(FixedArgs& a, int resident, int cap) {
+long long plan_slabs(FixedArgs& a, int sms, int per_sm, int cap) {
   const long long txy = (long long)a.tiles_x * a.tiles_y;
   const int nz = a.nz;
   if (txy <= 0 || nz <= 0) {
     a.nslab = 0;
     return 0;
   }
-  const long long res = resident > 0 ? resident : 1;
-  constexpr int kMinPlanes = 8;
+  const long long n_sm = sms > 0 ? sms : 1;
+  const long long res = n_sm * (per_sm > 0 ? per_sm : 1);
+  const long long fill = (txy * nz + 2 * n_sm - 1) / (2 * n_sm);  // planes of two CTAs per SM
+  const int min_planes = fill < 3 ? 3 : (fill > 8 ? 8 : (int)fill);
   int z = 0, i = 0;
+  const long long per_tile = res / txy;  // slabs the GPU holds at once
+  if (cap <= 0 && per_tile >= 9 && nz >= 8 * per_tile && per_tile <= kMaxSlabs) {
+    for (; i < per_tile; ++i) a.slab_z[i] = (int)((long long)nz * i / per_tile);
+    z = nz;
+  }
   while (z < nz) {
     const int rem = nz - z;
     const int left = kMaxSlabs - i;
     long long h = (txy * rem + res - 1) / res;  // remaining planes per resident CTA
     if (cap > 0 && h > cap) h = cap;
-    if (h < kMinPlanes && (cap <= 0 || cap >= kMinPlanes)) h = kMinPlanes;
+    if (h < min_planes && (cap <= 0 || cap >= min_planes)) h = min_planes;
     if (h * left < rem) h = (rem + left - 1) / left;
     if (h > rem) h = rem;
     a.slab_z[i++] = z;

@@ -453,14 +453,25 @@ constexpr int shape_warps(int sh) {
   return (sh == kR4W16 || sh == kR4W16S) ? 16 : (sh >= kR8W4L ? 4 : 8);
 }
 
-// z-slabs of one k_advect_fixed launch for `resident` CTAs on the GPU at once:
-// every slab takes the remaining planes per resident CTA (at most cap if > 0),
-// at least 8 and as many as kMaxSlabs slabs need.  The first slabs fill the
-// GPU once with the longest runs (K warm-up planes per slab), the short last
-// ones even out the end.  Measured (512^3, K = 3, 8 x 4): 617 GCUPS against 609
-// for first slabs of a quarter of that height; 256^3 509 against 502.  Sets
-// a.nslab / a.slab_z; returns the CTA count.
-long long plan_slabs(FixedArgs& a, int resident, int cap);
+// z-slabs of one k_advect_fixed launch, per_sm CTAs on each of sms SMs at once.
+// Sets a.nslab / a.slab_z; returns the CTA count.  K warm-up planes per slab ask
+// for few, tall ones; an even end asks for short ones:
+// - 9 slabs or more fit the GPU at once, each 8 planes or more: that many equal
+//   ones, a single wave (at most a tenth of it empty).  8 x 4, us, against the
+//   shrinking slabs below, K = 2 / 3 / 4: 180^3 28.7 / 49.2 / 63.5 against 35.0 /
+//   55.3 / 69.9; 300 x 200 x 150 42.8 / 64.4 / 96.4 against 46.8 / 71.9 / 97.9;
+//   256^3 75.8 / 102 / 166 against 75.7 / 102 / 164.  With 7 slabs (288^3) the
+//   single wave is the slower one: 105 / 143 / 212 against 102 / 137 / 206.
+// - otherwise every slab takes the remaining planes per resident CTA (at most cap
+//   if > 0): the first ones fill the GPU once, the short last ones even out the
+//   end.  512^3, K = 3: 617 GCUPS against 609 for first slabs of a quarter of that
+//   height.
+// - no slab below 8 planes, or, where slabs of 8 give less than two CTAs per SM,
+//   below what gives two (3 at least): such a grid waits for one CTA's march.  4 x 4, us per launch, K = 2 / 3 / 4: 64^3 with slabs of 4 8.2 /
+//   10.2 / 11.2 against 10.1 / 10.9 / 12.3; 48^3 of 3 6.2 / 8.2 / 8.2 against 8.2
+//   / 10.3 / 12.3; 96^3 of 4 12.3 / 16.4 / 20.5 against 12.3 / 16.0 / 18.5.
+// - at most kMaxSlabs.
+long long plan_slabs(FixedArgs& a, int sms, int per_sm, int cap);
 
 // 32-bit byte offsets for the shapes of the automatic choice at K <= 3, where
 // they measured faster (512^3, 8 x 4, GCUPS: K = 2 553 -> 580, K = 3 617 -> 636,
@@ -484,7 +495,7 @@ void launch_k(int cap, const int64_t* in, int64_t* out, FixedArgs a, cudaStream_
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long blocks = plan_slabs(a, per_sm * (sms > 0 ? sms : 1), cap);
+  const long long blocks = plan_slabs(a, sms, per_sm, cap);
   if (blocks <= 0) return;
   launch_dependent(kern, (unsigned)blocks, 32 * W, smem, st, in, out, a);  // cudaGetLastError: caller
 }
