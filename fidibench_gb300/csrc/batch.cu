@@ -170,6 +170,10 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
       sl[(b + 1) % 3].s = s;
       sl[(b + 1) % 3].kind = 1;
     }
+    auto scale = [s, d](int* s_to, int* d_to) {
+      *s_to = s;
+      *d_to = d;
+    };
     // this thread's rectangle of the packed tile (lanes and warps past the
     // last full rectangle join the last one, beyond its outputs)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -186,7 +190,7 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
     auto tile = [&](auto full, int levels, bool out_f64) {
       fx::advance_tile<K, R, W, true, fx::kLoadL2Regs, decltype(full)::value, false, kLeft, true,
                        kOff32>(
-          s_a, s_lev, 0, 0, 0, it.nout, levels, b == 0, out_f64, s, d, in, out, s_dyn, s_row,
+          s_a, s_lev, 0, 0, 0, it.nout, levels, b == 0, out_f64, scale, in, out, s_dyn, s_row,
           my_or, grp, lane - col * it.gw, (warp - rg * it.gh) * R);
     };
     if (b == nblocks - 1)
