@@ -864,6 +864,12 @@ int run_looped(fdb_batch* b, int steps, const double* dt, int K) {
 // to 340); from q = 400 on whole columns are best.  Measured, advect GCUPS,
 // depth 2, 4 rows and whole columns -> this: 8 x 96^3 99 -> 271; 40 x 64^3
 // 200 -> 375; 33 instances of [61, 98]^3 211 -> 349; 64 x 128^3 465 -> 496.
+//
+// Batches whose tiles of 8 planes at depth 4 fill at most half of the resident
+// CTAs wait for one tile after the other, block by block: the fewest blocks win.
+// 40 steps, us, rule above -> depth 4: 8 of [24, 40]^3 271 -> 237; 8 of [40, 64]^3
+// 345 -> 325; 4 x 48^3 339 -> 255; 4 x 64^3 360 -> 304.  Beyond half it loses: 4 x
+// 96^3 (576 tiles) 502 -> 512, 12 of [64, 90]^3 738 -> 794.
 void choose_tuning(fdb_batch* b) {
   struct Cand {
     int K, shape;
@@ -887,6 +893,16 @@ void choose_tuning(fdb_batch* b) {
   };
   double best = 0.0;
   std::vector<ItemDev> items;
+  const Variant* deep = find_variant(4, fx::kR4W8S, wide_planes(b));
+  if (deep && (b->K <= 0 || b->K == 4) && (b->shape < 0 || b->shape == fx::kR4W8S) && b->tz <= 0) {
+    pack({4, fx::kR4W8S}, 8, &items);
+    if (2 * (int)items.size() <= deep->resident()) {
+      b->eff_K = 4;
+      b->eff_shape = fx::kR4W8S;
+      b->eff_tz = 8;
+      return;
+    }
+  }
   for (const Cand& c : list) {
     int tz = b->tz;
     if (tz <= 0) {
