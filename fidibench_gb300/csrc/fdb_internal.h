@@ -176,13 +176,11 @@ struct FixedTuning {
 struct CoeffCarry {
   int64_t r[3] = {0, 0, 0};
 };
-int launch_advect_fixed(const Geom& g, const Coeffs3& c, int steps, int depth,
-                        double** buf, int* cur, double* d_scratch, size_t scratch_bytes,
-                        cudaStream_t s);
 // The scale pre-pass: slot ring reset, slot 0 = max|f| (FP64 bits) of the
 // geometry's own planes of f.
 int launch_scale_prepass(const Geom& g, const double* f, double* d_scratch, cudaStream_t s);
-// As above; *scale_slot (in/out, may be null) names the scratch slot that
+// `steps` steps by the fixed-point kernel; flips *cur once per launch.
+// *scale_slot (in/out, may be null) names the scratch slot that
 // holds max|f| of the current field (-1: unknown, a pre-pass measures it).
 int launch_advect_fixed_ex(const Geom& g, const Coeffs3& c, int steps, const FixedTuning& tune,
                            double** buf, int* cur, double* d_scratch, size_t scratch_bytes,

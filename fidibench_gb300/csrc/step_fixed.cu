@@ -387,13 +387,6 @@ uint64_t* scale_word(double* d_scratch, int i) {
   return reinterpret_cast<uint64_t*>(&((ScaleSlot*)d_scratch + (i % 3))->m);
 }
 
-int launch_advect_fixed(const Geom& g, const Coeffs3& c, int steps, int depth, double** buf,
-                        int* cur, double* d_scratch, size_t scratch_bytes, cudaStream_t s) {
-  FixedTuning t;
-  t.depth = depth;
-  return launch_advect_fixed_ex(g, c, steps, t, buf, cur, d_scratch, scratch_bytes, nullptr, s);
-}
-
 int launch_advect_fixed_ex(const Geom& g, const Coeffs3& c, int steps, const FixedTuning& tune,
                            double** buf, int* cur, double* d_scratch, size_t scratch_bytes,
                            int* scale_slot, cudaStream_t s) {
