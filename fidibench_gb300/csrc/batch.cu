@@ -950,8 +950,41 @@ void free_batch_adjoint(fdb_batch* b) {
   b->adj_scratch_bytes = 0;
 }
 
-// instance i between the caller's order and the stored order (see k_permute3)
+// Whether a kernel on the current device may read and write p (a copy may also
+// reach another GPU's memory).  FDB_FAULT=foreign denies it for every pointer but
+// the batch's own.
+bool on_current_device(const void* p) {
+  if (fault_injected("foreign")) return false;
+  int dev = 0;
+  cudaPointerAttributes at{};
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return (at.type == cudaMemoryTypeDevice && at.device == dev) || at.type == cudaMemoryTypeManaged;
+}
+
+// Whether p lies in one of the batch's own field buffers.
+bool own_memory(const fdb_batch* b, const void* p) {
+  const struct {
+    const double* at;
+    uint64_t cells;
+  } bufs[] = {{b->arena[0], (uint64_t)b->total},   {b->arena[1], (uint64_t)b->total},
+              {b->adj_lam[0], (uint64_t)b->total}, {b->adj_lam[1], (uint64_t)b->total},
+              {b->adj_io[0], (uint64_t)b->total},  {b->adj_io[1], (uint64_t)b->total},
+              {b->adj_user, (uint64_t)b->total},   {b->d_stage, b->stage_cells}};
+  const uintptr_t x = (uintptr_t)p;
+  for (const auto& m : bufs)
+    if (m.at && x >= (uintptr_t)m.at && x < (uintptr_t)(m.at + m.cells)) return true;
+  return false;
+}
+
+// instance i between the caller's order and the stored order (see k_permute3);
+// src and dst are memory that a kernel may use
 int launch_permute(fdb_batch* b, int i, const double* src, double* dst, bool to_view) {
+  for (const void* p : {(const void*)src, (const void*)dst})
+    if (!own_memory(b, p) && !on_current_device(p))
+      return fail(FDB_ERR_INVALID, "permutation of memory that the current device cannot reach");
   uint64_t n3[3];
   double v3[3], L3[3];
   view3(b->geoms_ref[i], n3, v3, L3);
@@ -993,18 +1026,6 @@ int make_io_table(fdb_batch* b) {
   return FDB_OK;
 }
 
-// Whether a kernel on the current device may read and write p (a copy may also
-// reach another GPU's memory).
-bool on_current_device(const void* p) {
-  int dev = 0;
-  cudaPointerAttributes at{};
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return (at.type == cudaMemoryTypeDevice && at.device == dev) || at.type == cudaMemoryTypeManaged;
-}
-
 // Cells of the caller's concatenated fields.
 uint64_t user_cells(const fdb_batch* b) {
   uint64_t c = 0;
@@ -1014,7 +1035,8 @@ uint64_t user_cells(const fdb_batch* b) {
 
 // Every instance between the caller's concatenated fields (device memory) and
 // an arena, on the batch's stream: one launch, or instance by instance where
-// the table does not serve.
+// the table does not serve or the caller's memory is another GPU's, which only
+// copies reach: a permuted instance then passes through d_stage.
 int io_all(fdb_batch* b, const double* src, double* dst, bool to_view) {
   if (b->d_io && on_current_device(to_view ? dst : src)) {
     const uint32_t blocks = std::min<uint32_t>(b->io_items, 152 * 8);
@@ -1028,10 +1050,14 @@ int io_all(fdb_batch* b, const double* src, double* dst, bool to_view) {
   for (int i = 0; i < b->count; ++i) {
     const double* s = src + (to_view ? b->offsets[i] : (int64_t)user);
     double* d = dst + (to_view ? (int64_t)user : b->offsets[i]);
-    if (b->permuted[i])
-      FDB_TRY(launch_permute(b, i, s, d, to_view));
-    else
-      FDB_CUDA_TRY(cudaMemcpyAsync(d, s, b->sizes[i] * 8, cudaMemcpyDeviceToDevice, b->stream));
+    const bool perm = b->permuted[i];
+    if (perm && to_view) {
+      FDB_TRY(launch_permute(b, i, s, b->d_stage, true));
+      s = b->d_stage;
+    }
+    FDB_CUDA_TRY(cudaMemcpyAsync(perm && !to_view ? b->d_stage : d, s, b->sizes[i] * 8,
+                                 cudaMemcpyDeviceToDevice, b->stream));
+    if (perm && !to_view) FDB_TRY(launch_permute(b, i, b->d_stage, d, false));
     user += b->sizes[i];
   }
   return FDB_OK;
