@@ -178,7 +178,13 @@ int launch_vel_contract(int count, const Geom* geoms, const int64_t* offsets, co
                         const double* lam, double* d_out, DeviceScratch& scratch,
                         cudaStream_t s) {
   if (count <= 0) return FDB_OK;
-  std::vector<ContractDev> insts(count);
+  // the copy's source lives in `scratch`: the stream may read it after this call,
+  // whose caller clears it behind its own wait (left over: that call failed)
+  std::vector<char>& table = scratch.host;
+  if (!table.empty()) FDB_CUDA_TRY(cudaStreamSynchronize(s));
+  const size_t b_insts = ((count * sizeof(ContractDev)) + 255) / 256 * 256;
+  table.assign(b_insts, 0);
+  ContractDev* insts = reinterpret_cast<ContractDev*>(table.data());
   std::vector<int> block_inst;
   int total = 0;
   for (int i = 0; i < count; ++i) {
@@ -204,7 +210,6 @@ int launch_vel_contract(int count, const Geom* geoms, const int64_t* offsets, co
     block_inst.insert(block_inst.end(), (size_t)nb, i);
     total += (int)nb;
   }
-  const size_t b_insts = ((count * sizeof(ContractDev)) + 255) / 256 * 256;
   const size_t b_table = ((total * sizeof(int)) + 255) / 256 * 256;
   const size_t need = b_insts + b_table + 3 * (size_t)total * sizeof(double);
   FDB_TRY(scratch.reserve(need));
@@ -212,11 +217,9 @@ int launch_vel_contract(int count, const Geom* geoms, const int64_t* offsets, co
   ContractDev* d_insts = (ContractDev*)base;
   int* d_table = (int*)(base + b_insts);
   double* d_part = (double*)(base + b_insts + b_table);
-  // pageable sources: the copies are staged before cudaMemcpyAsync returns
-  FDB_CUDA_TRY(cudaMemcpyAsync(d_insts, insts.data(), count * sizeof(ContractDev),
-                               cudaMemcpyHostToDevice, s));
-  FDB_CUDA_TRY(cudaMemcpyAsync(d_table, block_inst.data(), total * sizeof(int),
-                               cudaMemcpyHostToDevice, s));
+  const char* blocks = reinterpret_cast<const char*>(block_inst.data());
+  table.insert(table.end(), blocks, blocks + total * sizeof(int));
+  FDB_CUDA_TRY(cudaMemcpyAsync(base, table.data(), table.size(), cudaMemcpyHostToDevice, s));
   k_vel_contract<<<total, kThreads, 0, s>>>(f, lam, d_insts, d_table, d_part);
   k_vel_contract_finish<<<3 * count, kThreads, 0, s>>>(d_part, d_insts, d_out);
   note_launch(2);

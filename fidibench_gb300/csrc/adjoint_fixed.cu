@@ -881,6 +881,7 @@ int batch_adjoint_run(const BatchAdjointIO& io, cudaStream_t st) {
                                cudaMemcpyHostToDevice, st));
   FDB_CUDA_TRY(cudaMemcpyAsync(sc.guards, guards.data(), sizeof(int) * count,
                                cudaMemcpyHostToDevice, st));
+  FDB_CUDA_TRY(cudaStreamSynchronize(st));  // the sources end with this call
   FDB_CUDA_TRY(cudaMemsetAsync(sc.dpart, 0, sizeof(double) * 3 * grid, st));
   const unsigned eg = (unsigned)(count * kPerInst);
   const unsigned rg = (unsigned)((3 * count + 255) / 256);

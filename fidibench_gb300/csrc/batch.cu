@@ -766,13 +766,13 @@ int make_plan(fdb_batch* b, const double* dt, int K, int shape, int tz, bool tra
     FDB_TRY(balloc(&t->d_groups, groups.size()));
     t->group_cap = groups.size();
   }
-  // pageable sources: the copies are staged before cudaMemcpyAsync returns
   FDB_CUDA_TRY(cudaMemcpyAsync(t->d_insts, insts.data(), insts.size() * sizeof(InstDev),
                                cudaMemcpyHostToDevice, b->stream));
   FDB_CUDA_TRY(cudaMemcpyAsync(t->d_items, items.data(), items.size() * sizeof(ItemDev),
                                cudaMemcpyHostToDevice, b->stream));
   FDB_CUDA_TRY(cudaMemcpyAsync(t->d_groups, groups.data(), groups.size() * sizeof(fx::TileGroup),
                                cudaMemcpyHostToDevice, b->stream));
+  FDB_CUDA_TRY(cudaStreamSynchronize(b->stream));  // the sources end with this call
   t->shape = shape;
   t->tz = tz;
   t->dt.assign(dt, dt + b->count);
@@ -1022,6 +1022,7 @@ int make_io_table(fdb_batch* b) {
   FDB_TRY(balloc(&b->d_io, t.size()));
   FDB_CUDA_TRY(cudaMemcpyAsync(b->d_io, t.data(), t.size() * sizeof(IoDev),
                                cudaMemcpyHostToDevice, b->stream));
+  FDB_CUDA_TRY(cudaStreamSynchronize(b->stream));  // the source ends with this call
   b->io_items = (uint32_t)items;
   return FDB_OK;
 }
@@ -1451,6 +1452,7 @@ static int batch_adjoint_closed_form(fdb_batch* b, int S, const double* dt,
   FDB_CUDA_TRY(cudaMemcpyAsync(dda.data(), b->adj_dda, dda.size() * 8, cudaMemcpyDeviceToHost,
                                b->stream));
   FDB_TRY(bsync(b));
+  b->contract.host.clear();
   for (double& x : dda) x *= (double)S;
   batch_velocity_grad(b, dt, dda.data(), grad_v);
   return FDB_OK;

@@ -403,6 +403,7 @@ int adjoint_closed_form(fdb_upwind* h, int S, double dt, int arith, const double
   FDB_CUDA_TRY(cudaMemcpyAsync(h->hscal, h->dscal, 3 * sizeof(double), cudaMemcpyDeviceToHost,
                                h->stream));
   FDB_TRY(sync(h));
+  h->contract.host.clear();
   float ms = 0.f;
   h->adj_ms[0] = h->adj_ms[1] = h->adj_ms[2] = 0.0;
   if (cudaEventElapsedTime(&ms, t1.e, t2.e) == cudaSuccess) h->adj_ms[0] = ms;

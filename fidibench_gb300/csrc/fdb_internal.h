@@ -220,6 +220,7 @@ int launch_adjoint_finish(const double* dpart, double* d_out3, cudaStream_t s);
 struct DeviceScratch {
   void* ptr = nullptr;
   size_t bytes = 0;
+  std::vector<char> host;  // source of an upload into it, until the stream is waited for
   int reserve(size_t need);
   void release();
 };
@@ -227,7 +228,8 @@ struct DeviceScratch {
 // The velocity contraction of the closed-form adjoint (adjoint.cu): for each
 // instance i (geometry geoms[i], cells at offsets[i] of f and lam),
 // d_out[3 i + k] = sum_c lam[c] (f[c + up_k e_k] - f[c]) over the internal
-// axes k = z, y, x.  Deterministic; two launches.
+// axes k = z, y, x.  Deterministic; two launches.  The caller clears scratch.host
+// once it has waited for the stream.
 int launch_vel_contract(int count, const Geom* geoms, const int64_t* offsets, const double* f,
                         const double* lam, double* d_out, DeviceScratch& scratch,
                         cudaStream_t s);
