@@ -208,7 +208,7 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
 // cleared by k_batch_reset).  Block b works on instance b / per_inst; four loads
 // in flight per thread.
 __global__ void __launch_bounds__(256)
-k_batch_absmax(const double* __restrict__ arena, const int64_t* __restrict__ offs,
+k_batch_absmax(const double* arena, const int64_t* __restrict__ offs,
                const uint64_t* __restrict__ sizes, int per_inst, ScaleSlot* slots) {
   __shared__ unsigned long long sh[8];
   const int i = blockIdx.x / per_inst;

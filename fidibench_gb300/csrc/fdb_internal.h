@@ -41,7 +41,11 @@ void note_launch(uint64_t n = 1);
 // Programmatic dependent launch: the kernel's CTAs start while the last ones of
 // the launch before finish, and wait for its end in
 // cudaGridDependencySynchronize, before their first load.  A chain of short
-// launches takes 1.7 us each, the host's own time, instead of 4.1.
+// launches takes 1.7 us each, the host's own time, instead of 4.1.  Such a kernel
+// reads what the launch before wrote by ordinary (or L2) loads through pointers
+// without __restrict__: the read-only path (__ldg, or what the compiler makes of
+// const __restrict__) is for memory that nothing writes from the kernel's start
+// on, and its loads may be moved above the wait.
 template <typename... P, typename... A>
 cudaError_t launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
                              cudaStream_t s, A... args) {

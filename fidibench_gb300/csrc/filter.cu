@@ -91,7 +91,7 @@ constexpr int kFThreads = 256;
 // there in the map order), the others do not.
 template <int NT, bool CENTRE>
 __global__ void __launch_bounds__(kFThreads, 4)
-k_filter3(const double* __restrict__ in, double* __restrict__ out, const FArgs3 a) {
+k_filter3(const double* in, double* __restrict__ out, const FArgs3 a) {
   __shared__ double s_slots[kFThreads];
   const fdb::RegLoader reg(s_slots);
   const fdb::F64Regs f64(reg);
@@ -133,10 +133,10 @@ k_filter3(const double* __restrict__ in, double* __restrict__ out, const FArgs3 
       double v[NT > 0 ? NT : 1];
       if (inside) {
 #pragma unroll
-        for (int k = 0; k < NT; ++k) v[k] = __ldg(in + (i + a.t[k].lin));
+        for (int k = 0; k < NT; ++k) v[k] = in[i + a.t[k].lin];
       } else {
 #pragma unroll
-        for (int k = 0; k < NT; ++k) v[k] = __ldg(in + wrapped(a.t[k]));
+        for (int k = 0; k < NT; ++k) v[k] = in[wrapped(a.t[k])];
       }
       acc = first(wr[0], a.t[0].fuse, v[0]);
 #pragma unroll
@@ -147,7 +147,7 @@ k_filter3(const double* __restrict__ in, double* __restrict__ out, const FArgs3 
           acc = add(acc, wr[k], a.t[k].fuse, v[k]);
       }
     } else {
-      auto load = [&](int k) { return __ldg(in + (inside ? i + a.t[k].lin : wrapped(a.t[k]))); };
+      auto load = [&](int k) { return in[inside ? i + a.t[k].lin : wrapped(a.t[k])]; };
       acc = first(a.t[0].w, a.t[0].fuse, load(0));
       for (int k = 1; k < nterms; ++k) acc = add(acc, a.t[k].w, a.t[k].fuse, load(k));
     }

@@ -77,7 +77,7 @@ struct Walk {
 // the loop.
 template <int ARITH, typename I>
 __global__ void __launch_bounds__(kThreads)
-k_step3(const double* __restrict__ in, double* __restrict__ out, int64_t ntot, Walk<I> az,
+k_step3(const double* in, double* __restrict__ out, int64_t ntot, Walk<I> az,
         Walk<I> ay, Walk<I> ax, const Coeffs3 coeffs) {
   __shared__ double s_slots[kThreads];
   const RegLoader reg(s_slots);
@@ -134,7 +134,7 @@ struct SmallDiv {
 
 template <int ARITH>
 __global__ void __launch_bounds__(kTileThreads)
-k_steps_tile(const double* __restrict__ in, double* __restrict__ out, const TileArgs a,
+k_steps_tile(const double* in, double* __restrict__ out, const TileArgs a,
              const Coeffs3 coeffs) {
   extern __shared__ double s_buf[];
   __shared__ double s_slots[kTileThreads];

@@ -76,7 +76,7 @@ using fx::kMaxDepth;
 // max|f| as the bit pattern of |f| (monotone for non-negative doubles; NaN
 // and Inf patterns exceed every finite one) -> slot {m, kind 0}.
 __global__ void __launch_bounds__(256)
-k_absmax_bits(const double* __restrict__ f, uint64_t n, ScaleSlot* __restrict__ slot) {
+k_absmax_bits(const double* f, uint64_t n, ScaleSlot* slot) {
   __shared__ unsigned long long sh[8];
   unsigned long long m = 0ull;
   cudaGridDependencySynchronize();

@@ -124,8 +124,9 @@ __device__ __forceinline__ bool scale_from_slot(const ScaleSlot* slot, int guard
 // no other CTA writes the input during the launch), or L1-bypassing register
 // loads (the persistent batched kernel reads data that other CTAs wrote
 // earlier in the same launch, which L1 may hold stale).
-// kLoadRegs: read-only-path register loads one plane ahead (one tile per
-// launch, like cp.async, but without the shared-memory staging).
+// kLoadRegs: ordinary register loads one plane ahead (one tile per launch, like
+// cp.async, but without the shared-memory staging; not the read-only path, see
+// launch_dependent).
 enum Loader { kLoadCpAsync = 0, kLoadL2Regs = 1, kLoadRegs = 2 };
 
 // One rectangle of a packed tile (the persistent batched kernel): the output
@@ -172,8 +173,8 @@ template <int K, int R, int W, bool HSM, int LOADER, int FULL, bool STORE_G = fa
           bool LEFT_SMEM = false, bool GROUPED = false, bool OFF32 = false, class Scale>
 __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoeffs& lev, int tile_x, int tile_y, int Z0,
                                              int nout, int levels, bool in_f64, bool out_f64, Scale scale,
-                                             const int64_t* __restrict__ in,
-                                             int64_t* __restrict__ out, int64_t* s_dyn,
+                                             const int64_t* in, int64_t* __restrict__ out,
+                                             int64_t* s_dyn,
                                              int64_t (*s_row)[W][32],
                                              unsigned long long& my_or,
                                              const TileGroup& grp = TileGroup{}, int xlane = 0,
@@ -254,7 +255,7 @@ __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoef
     } else {
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        pre[r] = LOADER == kLoadRegs ? __ldg(at(src, r)) : __ldcg(at(src, r));
+        pre[r] = LOADER == kLoadRegs ? *at(src, r) : __ldcg(at(src, r));
     }
   }
 
@@ -283,7 +284,7 @@ __device__ __forceinline__ void advance_tile(const FixedArgs& a, const LevelCoef
         const int64_t* src = in + po_next;
 #pragma unroll
         for (int r = 0; r < R; ++r)
-          pre[r] = LOADER == kLoadRegs ? __ldg(at(src, r)) : __ldcg(at(src, r));
+          pre[r] = LOADER == kLoadRegs ? *at(src, r) : __ldcg(at(src, r));
       }
     }
     if (in_f64) {
@@ -399,7 +400,7 @@ __device__ __forceinline__ void cta_or(unsigned long long my_or, unsigned long l
 template <int K, int R, int W, bool HSM, int MINB, bool IN_F64, bool OUT_F64, bool STORE_G = false,
           int LOAD = kLoadCpAsync, bool LEFT = false, bool OFF32 = false>
 __global__ void __launch_bounds__(32 * W, MINB)
-k_advect_fixed(const int64_t* __restrict__ in, int64_t* __restrict__ out, const FixedArgs a) {
+k_advect_fixed(const int64_t* in, int64_t* __restrict__ out, const FixedArgs a) {
   extern __shared__ __align__(16) int64_t s_dyn[];
   __shared__ int64_t s_row[2][W][32];
   __shared__ unsigned long long s_or[W];
