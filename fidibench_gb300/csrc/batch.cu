@@ -37,7 +37,9 @@
 // An advect is three launches (counter and scale-ring reset, per-instance max|f|
 // pre-pass, persistent kernel), each dependent on the one before.  The device
 // tables of the plan stay until the tuning, a time step or a velocity changes;
-// the forward and the transposed problem have their own.
+// the forward and the transposed problem have their own.  A caller may capture an
+// advect whose tables are there: the batch then keeps those tables to its end and
+// its fields in the same arena.
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -598,8 +600,10 @@ const Variant* find_variant(int K, int shape, bool wide) {
 using namespace fdb;
 using namespace fdb::bt;
 
-// A plan and its device tables.
+// A plan and its device tables.  captured: a graph of the caller holds their
+// addresses, so that they are neither rewritten nor freed before the batch is.
 struct PlanTables {
+  bool captured = false;
   const Variant* v = nullptr;  // null: no plan
   int shape = -1, tz = 0;
   std::vector<double> dt;
@@ -638,6 +642,10 @@ struct fdb_batch {
   double* arena[2] = {nullptr, nullptr};
   int cur = 0;
   PlanTables tables[2];  // the forward problem's, the transposed one's
+  std::vector<void*> retired;  // tables of captured advects whose plan was replaced
+  // an advect was captured: from then on every advect leaves the fields in the
+  // arena it found them in, which is the one the caller's graph reads and writes
+  bool captured = false;
   ScaleSlot* d_slots = nullptr;
   unsigned* d_done = nullptr;
   unsigned* d_queue = nullptr;
@@ -710,6 +718,13 @@ bool wide_planes(const fdb_batch* b) {
   return false;
 }
 
+int is_capturing(fdb_batch* b, bool* yes) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  FDB_CUDA_TRY(cudaStreamIsCapturing(b->stream, &st));
+  *yes = st != cudaStreamCaptureStatusNone;
+  return FDB_OK;
+}
+
 // The plan of an advect with these settings into `t` (kept from the last call if
 // nothing changed): tiles, instance arguments, their device copies.  transposed:
 // every upwind direction reversed, the coefficients unchanged.
@@ -746,11 +761,16 @@ int make_plan(fdb_batch* b, const double* dt, int K, int shape, int tz, bool tra
   }
   if (groups.size() >= (1ull << 31))
     return fail(FDB_ERR_UNSUPPORTED, "batched plan exceeds 2^31 tile rectangles");
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  FDB_CUDA_TRY(cudaStreamIsCapturing(b->stream, &capturing));
-  if (capturing != cudaStreamCaptureStatusNone)
+  bool capturing = false;
+  FDB_TRY(is_capturing(b, &capturing));
+  if (capturing)
     return fail(FDB_ERR_CUDA, "a batched advect with new settings cannot be captured (its tables "
                               "are copied from the host): run it once before the capture");
+  if (t->captured) {
+    for (void* p : {(void*)t->d_insts, (void*)t->d_items, (void*)t->d_groups})
+      b->retired.push_back(p);
+    *t = PlanTables();
+  }
   if (!t->d_insts) FDB_TRY(balloc(&t->d_insts, (size_t)b->count));
   if (items.size() > t->item_cap) {
     if (t->d_items) cudaFree(t->d_items);
@@ -789,6 +809,8 @@ int run_batched(fdb_batch* b, int steps, const double* dt, int K, int shape, int
   const int nblocks = (steps + K - 1) / K;
   if ((int64_t)nblocks * t.ipb >= (1ll << 31))
     return fail(FDB_ERR_UNSUPPORTED, "batched work queue exceeds 2^31 items");
+  bool capturing = false;
+  FDB_TRY(is_capturing(b, &capturing));
   const int grid = (int)std::min<int64_t>((int64_t)nblocks * t.ipb, t.resident);
   cudaStream_t st = b->stream;
   k_batch_reset<<<(3 * b->count + 255) / 256, 256, 0, st>>>(b->d_slots, b->d_done, b->d_queue,
@@ -809,7 +831,13 @@ int run_batched(fdb_batch* b, int steps, const double* dt, int K, int shape, int
                       inject ? 2000000ll : kWaitCycles, st));
   note_launch(3);
   FDB_CUDA_TRY(cudaGetLastError());
-  b->cur ^= (nblocks & 1);
+  if (capturing) t.captured = b->captured = true;
+  // an odd number of blocks ends in the other arena; the transposed steps run on
+  // the adjoint buffers, which no graph holds (their calls wait for the stream)
+  if (!b->captured || transposed)
+    b->cur ^= (nblocks & 1);
+  else if (nblocks & 1)
+    FDB_CUDA_TRY(cudaMemcpyAsync(a0, a1, (size_t)b->total * 8, cudaMemcpyDeviceToDevice, st));
   return FDB_OK;
 }
 
@@ -817,8 +845,8 @@ int run_batched(fdb_batch* b, int steps, const double* dt, int K, int shape, int
 // K steps per fixed-point launch; K <= 0: what fdb_upwind_advect runs for
 // each instance (the fixed kernel at its default depth where it is
 // supported and preferred, the FP64 kernel otherwise).  Every instance ends
-// in the same arena: the one most instances end in; the others are copied
-// across.
+// in the same arena: the one most instances end in (once captured: the one they
+// began in); the others are copied across.
 int run_looped(fdb_batch* b, int steps, const double* dt, int K) {
   const size_t per = (fixed_scratch_bytes() + 7) / 8;
   std::vector<int> fin(b->count);
@@ -842,7 +870,10 @@ int run_looped(fdb_batch* b, int steps, const double* dt, int K) {
   }
   int ones = 0;
   for (int i = 0; i < b->count; ++i) ones += fin[i];
-  const int new_cur = 2 * ones > b->count ? 1 : 0;
+  bool capturing = false;
+  FDB_TRY(is_capturing(b, &capturing));
+  b->captured |= capturing;
+  const int new_cur = b->captured ? b->cur : 2 * ones > b->count ? 1 : 0;
   for (int i = 0; i < b->count; ++i) {
     if (fin[i] == new_cur) continue;
     FDB_CUDA_TRY(cudaMemcpyAsync(b->arena[new_cur] + b->offsets[i], b->arena[fin[i]] + b->offsets[i],
@@ -1181,6 +1212,7 @@ int fdb_batch_destroy(fdb_batch* b) {
     cudaFree(t.d_items);
     cudaFree(t.d_groups);
   }
+  for (void* p : b->retired) cudaFree(p);
   free_batch_adjoint(b);
   b->contract.release();
   if (b->h_sums) cudaFreeHost(b->h_sums);

@@ -294,8 +294,16 @@ int fdb_upwind_adjoint_step(fdb_upwind* h, double dt, const double* f_dev,
  * (upwind.cxx:23-49) with ndims <= 3, advanced together.
  * fdb_batch_advect runs one persistent launch per call (all instances, all
  * time blocks, per-instance dependency tracking with bounded waits; its tables
- * are kept while dt, the velocities and the tuning stay the same, and have to
- * be there before the call is captured into a CUDA graph).
+ * are kept while dt, the velocities and the tuning stay the same).
+ * A caller may capture it into a CUDA graph on the batch's stream, once a call
+ * with the same dt, velocities, tuning and stream has run outside of the capture
+ * (FDB_ERR_CUDA otherwise).  The capture itself advances nothing; each replay
+ * advances the batch's fields, whatever they are by then, by num_steps with the
+ * dt, velocities and tuning of the capture, also after later calls with others.
+ * Replays and other calls on the batch have to be ordered on its stream, and
+ * fdb_batch_destroy ends the graph's validity.  A captured batch keeps the
+ * tables of every captured plan until then, and its advects with an odd number
+ * of time blocks copy the fields back.
  * fdb_batch_advect_looped is the comparator: the single-field kernel looped
  * over the instances, with the depth set by FDB_TUNE_DEPTH (equal depths
  * give bit-identical fields) or, without one, each instance's single-field
