@@ -54,6 +54,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "batch_max.h"
 #include "step_fixed.cuh"
 
 using fdb::fx::FixedArgs;
@@ -207,43 +208,53 @@ k_batch_fixed(const InstDev* __restrict__ insts, const ItemDev* __restrict__ ite
 }
 
 // max|f| of every instance (FP64 bit patterns) into slot 0 of its ring (kind 0,
-// cleared by k_batch_reset).  Block b works on instance b / per_inst; four loads
-// in flight per thread.
+// cleared by k_batch_reset), one chunk of cells per block (max_chunks) and four
+// loads in flight per thread.  Bound by HBM: 256 instances (223 M cells) 257 us,
+// 6.9 TB/s; 512^3 beside 2000 of 8^3 166 us, 6.5 TB/s.
 __global__ void __launch_bounds__(256)
 k_batch_absmax(const double* arena, const int64_t* __restrict__ offs,
-               const uint64_t* __restrict__ sizes, int per_inst, ScaleSlot* slots) {
+               const uint64_t* __restrict__ sizes, const uint64_t* __restrict__ first, int count,
+               uint64_t cells, ScaleSlot* slots) {
   __shared__ unsigned long long sh[8];
-  const int i = blockIdx.x / per_inst;
-  const int part = blockIdx.x - i * per_inst;
-  const double* f = arena + offs[i];
-  const uint64_t n = sizes[i];
-  const uint64_t step = (uint64_t)per_inst * 256;
+  const uint64_t chunks = first[count];
   cudaGridDependencySynchronize();
-  unsigned long long m = 0ull;
-  auto take = [&](double x) {
-    const unsigned long long bits =
-        (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
-    m = bits > m ? bits : m;
-  };
-  uint64_t k = (uint64_t)part * 256 + threadIdx.x;
-  for (; k + 3 * step < n; k += 4 * step) {
-    const double x0 = f[k], x1 = f[k + step], x2 = f[k + 2 * step], x3 = f[k + 3 * step];
-    take(x0);
-    take(x1);
-    take(x2);
-    take(x3);
-  }
-  for (; k < n; k += step) take(f[k]);
+  for (uint64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+    int i = 0, hi = count;  // the instance whose chunks contain this one
+    while (hi - i > 1) {
+      const int mid = (i + hi) >> 1;
+      if (first[mid] <= c) i = mid;
+      else hi = mid;
+    }
+    const double* f = arena + offs[i];
+    const uint64_t begin = (c - first[i]) * cells;
+    const uint64_t end = min(sizes[i], begin + cells);
+    unsigned long long m = 0ull;
+    auto take = [&](double x) {
+      const unsigned long long bits =
+          (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+      m = bits > m ? bits : m;
+    };
+    uint64_t k = begin + threadIdx.x;
+    for (; k + 3 * 256 < end; k += 4 * 256) {
+      const double x0 = f[k], x1 = f[k + 256], x2 = f[k + 512], x3 = f[k + 768];
+      take(x0);
+      take(x1);
+      take(x2);
+      take(x3);
+    }
+    for (; k < end; k += 256) take(f[k]);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
-    m = v > m ? v : m;
-  }
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) m = sh[w] > m ? sh[w] : m;
-    atomicMax(&slots[3 * i].m, m);
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
+      m = v > m ? v : m;
+    }
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) m = sh[w] > m ? sh[w] : m;
+      atomicMax(&slots[3 * (int64_t)i].m, m);
+    }
+    __syncthreads();
   }
 }
 
@@ -652,6 +663,8 @@ struct fdb_batch {
   int* d_err = nullptr;
   int64_t* d_offs = nullptr;
   uint64_t* d_sizes = nullptr;
+  MaxChunks max;  // work items of the max|f| pass
+  uint64_t* d_max_first = nullptr;
   double* d_part = nullptr;
   double* d_sums = nullptr;
   double* h_sums = nullptr;
@@ -815,12 +828,10 @@ int run_batched(fdb_batch* b, int steps, const double* dt, int K, int shape, int
   cudaStream_t st = b->stream;
   k_batch_reset<<<(3 * b->count + 255) / 256, 256, 0, st>>>(b->d_slots, b->d_done, b->d_queue,
                                                             b->count);
-  // a wave of blocks over all instances, and the largest one's share per block short
-  const uint64_t largest = *std::max_element(b->sizes.begin(), b->sizes.end());
-  const int per_inst = (int)std::min<uint64_t>(
-      4096, std::max<uint64_t>({8, (uint64_t)(152 * 8 / b->count), largest / 32768}));
-  FDB_CUDA_TRY(launch_dependent(k_batch_absmax, (unsigned)(b->count * per_inst), 256, 0, st,
-                                b->arena[b->cur], b->d_offs, b->d_sizes, per_inst, b->d_slots));
+  const unsigned max_blocks = (unsigned)std::min<uint64_t>(b->max.first.back(), 0x7FFFFFFF);
+  FDB_CUDA_TRY(launch_dependent(k_batch_absmax, max_blocks, 256, 0, st, b->arena[b->cur],
+                                b->d_offs, b->d_sizes, b->d_max_first, b->count, b->max.cells,
+                                b->d_slots));
   int64_t* a0 = (int64_t*)b->arena[b->cur];
   int64_t* a1 = (int64_t*)b->arena[b->cur ^ 1];
   // FDB_FAULT=timeout makes every dependency unsatisfiable and the wait
@@ -1160,13 +1171,16 @@ int fdb_batch_create(int count, const fdb_instance_desc* descs, fdb_batch** out)
     return cuda_fail(e, "cudaStreamCreate");
   }
   b->stream = b->own;
+  b->max = max_chunks(b->sizes);
   const size_t per = (fixed_scratch_bytes() + 7) / 8;
   int rc = FDB_OK;
   if ((rc = balloc(&b->arena[0], b->total)) || (rc = balloc(&b->arena[1], b->total)) ||
       (rc = balloc(&b->d_slots, 3 * count)) ||
       (rc = balloc(&b->d_done, count)) || (rc = balloc(&b->d_queue, 1)) ||
       (rc = balloc(&b->d_err, 1)) || (rc = balloc(&b->d_offs, count)) ||
-      (rc = balloc(&b->d_sizes, count)) || (rc = balloc(&b->d_part, count * kSumPerInst)) ||
+      (rc = balloc(&b->d_sizes, count)) ||
+      (rc = balloc(&b->d_max_first, (size_t)count + 1)) ||
+      (rc = balloc(&b->d_part, count * kSumPerInst)) ||
       (rc = balloc(&b->d_sums, count)) || (rc = balloc(&b->d_plain_scratch, per * count)) ||
       (b->stage_cells && (rc = balloc(&b->d_stage, b->stage_cells)))) {
     fdb_batch_destroy(b);
@@ -1180,6 +1194,9 @@ int fdb_batch_create(int count, const fdb_instance_desc* descs, fdb_batch** out)
     e = cudaMemcpyAsync(b->d_offs, b->offsets.data(), count * 8, cudaMemcpyHostToDevice, b->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->d_sizes, b->sizes.data(), count * 8, cudaMemcpyHostToDevice, b->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(b->d_max_first, b->max.first.data(), (count + 1) * 8,
+                        cudaMemcpyHostToDevice, b->stream);
   if (e != cudaSuccess) {
     fdb_batch_destroy(b);
     return cuda_fail(e, "batch set-up");
@@ -1204,7 +1221,7 @@ int fdb_batch_destroy(fdb_batch* b) {
   drop_plans(b);
   void* ps[] = {b->arena[0], b->arena[1], b->d_slots,  b->d_done,  b->d_queue, b->d_err,    b->d_offs,
                 b->d_sizes,  b->d_part,  b->d_sums,  b->d_plain_scratch, b->d_stage,
-                b->d_io};
+                b->d_io, b->d_max_first};
   for (void* p : ps)
     if (p) cudaFree(p);
   for (PlanTables& t : b->tables) {

@@ -12,7 +12,7 @@ import re
 from conftest import ROOT
 
 # tables that the host has uploaded, and waited for, before the chain of launches
-TABLES = {"insts", "items", "groups", "offs", "sizes"}
+TABLES = {"insts", "items", "groups", "offs", "sizes", "first"}
 
 
 def _kernels():
