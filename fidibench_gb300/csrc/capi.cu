@@ -66,6 +66,15 @@ struct fdb_upwind {
   int chain_first = 0;
   int chain_K = 0;
   fdb::CoeffCarry chain_carry;  // coefficient errors carried from block to block
+  // the chain's last fixed-point block as it was launched (chain_settle)
+  struct {
+    int steps = 0;
+    bool in_f64 = false;
+    fdb::CoeffCarry carry;  // before it
+    fdb::Geom g;
+    fdb::Coeffs3 c;
+  } chain_prev;
+  bool chain_touched = false;  // the caller wrote planes or the scale word since
 };
 
 namespace fdb {
@@ -287,6 +296,35 @@ int advance(fdb_upwind* h, int steps, double dt, int arith) {
   }
   h->scale_slot = -1;
   return launch_advect_f64(g, c, arith, steps, h->buf, &h->cur, h->stream);
+}
+
+// Before a block with the coefficients c in an open fixed-point chain.  Earlier
+// blocks may have left a coefficient error to later ones (fixed_point.cuh), which
+// cancels to first order among equal steps only: where the coefficients change,
+// 2^-31 (a - a') D^2 f would stay.  The last block is then launched again as the
+// one that closes the chain (all 62 bits in its last step, FP64 out) and the chain
+// goes on from its field.  Planes or a scale word that the caller has written since
+// would be lost: refused.
+int chain_settle(fdb_upwind* h, const Coeffs3& c) {
+  const Geom& g = h->g;
+  auto& prev = h->chain_prev;
+  const CoeffCarry& r = h->chain_carry;
+  if (h->chain_first || !(r.r[0] || r.r[1] || r.r[2])) return FDB_OK;
+  if (c.az == prev.c.az && c.ay == prev.c.ay && c.ax == prev.c.ax && g.upz == prev.g.upz &&
+      g.upy == prev.g.upy && g.upx == prev.g.upx)
+    return FDB_OK;
+  if (h->chain_touched)
+    return fail(FDB_ERR_INVALID,
+                "the time step or velocity changed inside a fixed-point block chain whose planes or "
+                "scale word were exchanged: close the chain (last = 1) before the change and begin "
+                "another one");
+  h->cur ^= 1;
+  FDB_TRY(launch_fixed_block(prev.g, prev.c, prev.steps, h->tune, h->chain_K, h->buf, &h->cur,
+                             prev.in_f64, true, h->scratch, h->chain_i - 1, &prev.carry,
+                             h->stream));
+  h->chain_first = 1;
+  h->chain_carry = CoeffCarry();
+  return FDB_OK;
 }
 
 // A CUDA event that lives as long as its scope.
@@ -594,6 +632,7 @@ int fdb_upwind_set_planes(fdb_upwind* h, uint64_t first, uint64_t count, const d
   // the caller agrees the scale word instead)
   if (!h->chain) h->scale_slot = -1;
   if (len == 0) return FDB_OK;
+  h->chain_touched = true;
   FDB_CUDA_TRY(cudaMemcpyAsync(h->buf[h->cur] + off, src, len * sizeof(double),
                                is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                h->stream));
@@ -644,10 +683,15 @@ int fdb_upwind_advect_block(fdb_upwind* h, int steps, double dt, int last) {
   if (h->chain_arith == FDB_ARITH_FIXED) {
     if (steps > h->chain_K)
       return fail(FDB_ERR_INVALID, "a fixed-point block advances at most its depth of steps");
-    rc = launch_fixed_block(h->g, c, steps, h->tune, h->chain_K, h->buf, &h->cur,
-                            h->chain_first != 0, last != 0, h->scratch, h->chain_i,
-                            &h->chain_carry, h->stream);
+    rc = chain_settle(h, c);
+    if (rc == FDB_ERR_INVALID) return rc;  // the chain stays as it was
+    h->chain_prev = {steps, h->chain_first != 0, h->chain_carry, h->g, c};
+    if (!rc)
+      rc = launch_fixed_block(h->g, c, steps, h->tune, h->chain_K, h->buf, &h->cur,
+                              h->chain_first != 0, last != 0, h->scratch, h->chain_i,
+                              &h->chain_carry, h->stream);
     if (!rc) {
+      h->chain_touched = false;
       ++h->chain_i;
       h->chain_first = 0;
       if (last) h->scale_slot = h->chain_i % 3;
@@ -680,6 +724,7 @@ int fdb_upwind_set_scale_word(fdb_upwind* h, const uint64_t* src, int is_device)
   if (!src) return fail(FDB_ERR_INVALID, "null source");
   if (!h->chain || h->chain_arith != FDB_ARITH_FIXED)
     return fail(FDB_ERR_INVALID, "no fixed-point block chain is open");
+  h->chain_touched = true;
   FDB_CUDA_TRY(cudaMemcpyAsync(scale_word(h->scratch, h->chain_i), src, sizeof(uint64_t),
                                is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                h->stream));
@@ -750,6 +795,7 @@ int fdb_upwind_field_ptr(fdb_upwind* h, double** out) {
   if (!out) return fail(FDB_ERR_INVALID, "null output pointer");
   *out = h->buf[h->cur];
   h->scale_slot = -1;  // the caller may write through the pointer
+  h->chain_touched = true;
   return FDB_OK;
 }
 

@@ -133,8 +133,9 @@ FDB_HD QCoeff step_qcoeff(const QCoeff& q, int64_t n, bool last) {
   return r;
 }
 
-// The same step by step, for steps whose coefficient may change: *carry (0
-// before the first step) is the error carried in, in units of 2^-62.
+// The same step by step: *carry (0 before the first step) is the error carried
+// in, in units of 2^-62.  The steps of one carry have equal coefficients, the
+// condition for their errors to cancel.
 inline QCoeff step_qcoeff_carry(const QCoeff& q, int64_t* carry, bool last) {
   const int64_t v = *carry + q.a0;
   const int64_t inc = (v + 0x80000000ll) >> 32;

@@ -164,6 +164,11 @@ int fdb_upwind_set_own_planes(fdb_upwind* h, uint64_t first, uint64_t count);
  * make every slab's scale word equal to the maximum over the slabs
  * (fdb_upwind_get/set_scale_word, device pointers, stream-ordered): then the
  * slabs of a grid advance with one scale, exactly as the whole grid would.
+ * dt is the chain's own.  A block under the fixed-point arithmetic with another
+ * dt or velocity is as if the chain had been closed before it and another one
+ * begun; once planes or the scale word have been written since the last block
+ * (a slab's halo), that is no longer possible and returns FDB_ERR_INVALID, the
+ * chain unchanged: there, close the chain before the change.
  * While a chain is open the calls that read or write the field as FP64
  * return FDB_ERR_INVALID.  No reference counterpart. */
 int fdb_upwind_block_begin(fdb_upwind* h, double dt, int* fixed);
