@@ -3,9 +3,9 @@
 //
 // A field value f is carried as the integer F = round(f * 2^s) for one scale
 // s shared by the whole launch (chosen from max|f| so that |F| < 2^60 / G^K,
-// G the step's max-norm growth bound).  Conversions are done with integer
-// operations on the IEEE-754 bit pattern (the FP64 pipe of GB300 retires only
-// ~2 conversions per clock per SM, the integer pipes ~64-128 operations).
+// G the step's max-norm growth bound).  f to F uses integer operations on the
+// IEEE-754 bit pattern; F to f is one conversion on the FP64 pipe, which the
+// integer work of the neighbouring cells covers (to_double).
 //
 // The update F' = F + sum_j a_j (F_up_j - F) multiplies 64-bit differences
 // D_j (|D_j| < 2^60) by coefficients a_j in [0, 1] held in Q1.62 (A = a 2^62),
@@ -29,10 +29,14 @@
 // S-1 therefore take the multiple of 2^-30 that carries the error of the steps
 // before it (dithered: |sum e| <= 2^-31 after every step), where a0 = 0 and
 // six products remain (fixed_update6), and step S takes the rest to 62 bits.
-// The remainder is S 2^-62 times a second difference of the field: below the
-// rounding of the S steps (2 units of F each), and the a0 d0 terms that the
-// nine-product form drops on every step (up to 6 units, with the sign of a0:
-// a drift of the mean) are dropped once.
+// The remainder, -1/2 sum_n (sum_j e_j,n D_j)^2 with sum_n e_j,n^2 <= (S / 4 + 1)
+// 2^-60, is at most 2.25 units of F per step (three axes, the highest frequency,
+// undamped), beside 2 units of rounding; the nine-product form's 2 units of
+// rounding come with up to 6 of the a0 d0 terms that it drops on every step, with
+// the sign of a0 (a drift of the mean), here dropped once.  Errors against 64 bits,
+// 1000 random problems (CFL 0.1 .. 0.5, 2 .. 200 steps), against nine products on
+// every step: geometric mean 0.20 times, the largest 6.4e-16 of max|f| instead of
+// 5.2e-14; larger in 3.6 % of them, 1.34 times at most.
 #pragma once
 
 #include <stdint.h>

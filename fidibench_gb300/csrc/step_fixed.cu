@@ -11,10 +11,11 @@
 //
 // Precision.  The scale keeps |F| < 2^(59-g) at a launch's input (g guard
 // bits cover the step's max-norm growth G^K), so one unit of F is at most
-// 2^-(58-g) of max|f|.  One step adds < 8 units of truncation error per cell,
-// so after 100 steps the field is within ~1e-15 of the reference's FP64
-// arithmetic relative to max|f| (the bar is 1e-13).  Cells below one unit
-// are held as 0, an absolute error below the same bound.
+// 2^-(58-g) of max|f|.  One step adds at most 2 units of rounding per cell (8
+// units in all on the last one) and 2.25 of the coefficients' remainder
+// (fixed_point.cuh), so after 100 steps the field is within ~1e-15 of the
+// reference's FP64 arithmetic relative to max|f| (the bar is 1e-13).  Cells below
+// one unit are held as 0, an absolute error below the same bound.
 //
 // Update.  F' = F + sum_j a_j (F_up_j - F) with a_j in [0, 1] held in Q1.62
 // (A = a1 2^32 + a0, a0 balanced to [-2^31, 2^31)).  For D = d1 2^32 + d0:

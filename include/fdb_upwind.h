@@ -53,7 +53,12 @@ extern "C" {
  *  FDB_ARITH_FIXED : temporally blocked kernel that carries the field in
  *                    64-bit block-fixed-point between one FP64 load and one
  *                    FP64 store per block of steps (integer pipes instead of
- *                    the FP64 pipe).
+ *                    the FP64 pipe).  The coefficients a_j = |c_j| have 62 bits
+ *                    on the last step of an advect and 30 on the others, whose
+ *                    errors are carried from step to step and sum to zero: with
+ *                    the rounding, a step that does not amplify adds at most
+ *                    7e-17 of max|f| to the error (the bound at the highest
+ *                    frequency; measured, 100 steps add up to 6e-16).
  *  FDB_ARITH_AUTO  : FIXED where the geometry allows it, else FMA (default). */
 #define FDB_ARITH_AUTO 0
 #define FDB_ARITH_EXACT 1
