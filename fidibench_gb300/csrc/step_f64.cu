@@ -318,9 +318,17 @@ int launch_steps_tile(const TileArgs& a, const Coeffs3& c, const double* in, dou
 template <typename I>
 cudaError_t step3(const Geom& g, const Coeffs3& c, int arith, const double* in, double* out,
            cudaStream_t s) {
-  // all CTAs resident at once, fewer for grids with less than a cell per thread
-  int64_t grid = ((int64_t)g.ntot + kThreads - 1) / kThreads;
-  if (grid > kSms * 8) grid = kSms * 8;
+  // The same number of cells for every CTA.  6 are resident per SM (38 to 40
+  // registers), and a dependent launch's first ones go to the SMs that the launch
+  // before leaves first: 8 per SM fall unevenly on the SMs, whole waves less so, where
+  // a thread still has a few cells.  FMA, us per step with 8 / 12 / 18 per SM: 512^3
+  // 1036 / 919 / 897, 4000 x 3000 94.6 / 84.1 / 83.5, 208^3 69.9 / 63.5 / 62.9, 192^3
+  // 55.7 / 49.9 / 50.7, 2048^2 30.3 / 30.0 / 30.4, 144^3 22.1 / 22.2 / 22.3, 128^3 16.6
+  // / 17.1 / 16.9 (normal launches of 8: 512^3 947, 2048^2 32.9).  EXACT 512^3 1978 /
+  // 1963 / 1955.
+  const int per_sm = g.ntot >= 8000000 ? 18 : g.ntot >= 3000000 ? 12 : 8;
+  int64_t grid = ((int64_t)g.ntot + kThreads - 1) / kThreads;  // a cell per thread at least
+  if (grid > kSms * per_sm) grid = kSms * per_sm;
   const int64_t stride = grid * kThreads;
   const int64_t dy = stride / g.nx;
   const Walk<I> ax = make_walk<I>(g.nx, 1, g.upx, stride % g.nx);
