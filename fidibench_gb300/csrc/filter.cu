@@ -248,7 +248,8 @@ int launch_apply(fdb_filter* f) {
   const int nt = (int)f->w.size();
   if (f->ndims <= 3 && nt <= kMaxFastTerms) {
     FArgs3 a{};
-    // all CTAs resident at once, fewer for grids with less than a cell per thread
+    // 8 CTAs per SM, the same number of cells for each: two even waves of 4 (60 to 64
+    // registers with 3 to 7 terms).  Fewer for grids with less than a cell per thread.
     long long blocks = std::min<long long>(((long long)f->ntot + kFThreads - 1) / kFThreads,
                                            152 * (2048 / kFThreads));
     long long rest = blocks * kFThreads;  // the grid stride, in digits of the extents

@@ -14,8 +14,8 @@
 // cost of an FP64 operation (f64_regs.cuh) and an even share of the cells for
 // every SM.  Per step, against rows dealt to CTAs and DADD / DMUL / DFMA with
 // constants: EXACT 192^3 133 -> 106 us (67 of the pipe's 67 cycles per
-// operation and warp), FMA 2048^2 38 -> 29.7 us, FMA 128^3 20.5 -> 15.8 us.
-// Small grids are bound by the launches: see plan_f64.
+// operation and warp), FMA 2048^2 38 -> 30.3 us, FMA 128^3 20.5 -> 16.5 us, FMA 512^3
+// 1490 -> 897 us (150 GCUPS).  Small grids are bound by the launches: see plan_f64.
 //
 // Layout: row-major, x (last reference axis) contiguous; consecutive threads
 // take consecutive cells, and the upstream neighbours come through L1 and L2.
@@ -319,9 +319,8 @@ template <typename I>
 cudaError_t step3(const Geom& g, const Coeffs3& c, int arith, const double* in, double* out,
            cudaStream_t s) {
   // The same number of cells for every CTA.  6 are resident per SM (38 to 40
-  // registers), and a dependent launch's first ones go to the SMs that the launch
-  // before leaves first: 8 per SM fall unevenly on the SMs, whole waves less so, where
-  // a thread still has a few cells.  FMA, us per step with 8 / 12 / 18 per SM: 512^3
+  // registers): of 8, the last two run nearly alone, and in a dependent launch they
+  // fall unevenly on the SMs.  Whole waves, where a thread still has a few cells.  FMA, us per step with 8 / 12 / 18 per SM: 512^3
   // 1036 / 919 / 897, 4000 x 3000 94.6 / 84.1 / 83.5, 208^3 69.9 / 63.5 / 62.9, 192^3
   // 55.7 / 49.9 / 50.7, 2048^2 30.3 / 30.0 / 30.4, 144^3 22.1 / 22.2 / 22.3, 128^3 16.6
   // / 17.1 / 16.9 (normal launches of 8: 512^3 947, 2048^2 32.9).  EXACT 512^3 1978 /
